@@ -124,7 +124,46 @@ struct TileGenParams {
     float vf[3][2][kMaxSeg], wf[3][2][kMaxSeg];
 };
 
-struct SigPlan;
+// Coefficients of the segment kinds of a LinePlan (0 first, 1 long interior, 2
+// short interior, 3 last segment; periodic lines use 1 and 2), kernel
+// parameters of k_line.  f: q = 1 -> l, 1/u0, u1/u0; q = 2 -> L1, L2, u1/u0,
+// u2/u0, 1/u0, with rows past the segment's end copying the forward values
+// upwards and contributing nothing backwards.  v / w: spikes.  tl: what the tail
+// needs (see ln_sweep).
+template <typename T, int Q, int MS>
+struct LineCoef {
+    T f[4][Q == 1 ? 3 : 5][MS];
+    T v[4][Q][MS], w[4][Q][MS];
+    T tl[4][4];
+    T clo[kMaxClo][kMaxCloLen], chi[kMaxClo][kMaxCloLen];   // closure rows, as in CompactParams
+    T ci[CLES_MAX_M], a0, pad_;
+};
+
+// Segmented form of a line of any length (k_line): S segments, the first `rem`
+// of base + 1 points and the others of base, on register tiles of MS points.
+struct LinePlan {
+    int MS = 32, S = 0, base = 0, rem = 0;
+    int mm = 0;                       // longest segment, rounded up to a group of four rows
+    int Wn = 0, Kr = 0;               // interface window: segments, radius
+    std::vector<unsigned char> coef;  // LineCoef<plan dtype, q, MS>
+    void* dcoef = nullptr;            // the same on the device
+    void* tab = nullptr;              // reduced inverse rows, [S][2q][Wn][2q], plan dtype
+    ~LinePlan();
+};
+struct LineArgs {
+    FieldView in, out;
+    int S, base, rem, mm, Wn, Kr;
+    int logL, SC, CL;                 // lines (log2) and segments per block, blocks per cluster
+    int pitch, kpad;                  // shared row of an x line: pitch, one pad element every 2^kpad
+    int gstage;                       // the block's inverse rows are staged in shared memory
+    int mode, rk_first;
+    struct {
+        double *Q, *du;
+        double A, B, dt;
+        const double* dtp;
+    } rk;
+};
+
 struct CompactPlan {
     bool has_tl = false;
     TileLineParams TL;
@@ -137,33 +176,8 @@ struct CompactPlan {
     double* tab64 = nullptr;
     float* tab32 = nullptr;
     size_t tab_elems = 0;
-    // few long closed x lines: the line is cut into pieces solved side by side
-    std::unique_ptr<SigPlan> sig;
+    std::unique_ptr<LinePlan> line;   // k_line form, where the plan has one
     ~CompactPlan();
-};
-
-// Few long closed x lines (1-D problems, very thin 2-D grids) split into P
-// pieces inside the GPU: the reference's P > 1 line solve (src/tridiag.jl:
-// 136-170, src/banded.jl:177-214) with the pieces of one line in place of
-// ranks and global memory in place of the exchange.  Pieces of one class
-// share a local plan: the first (closed low end, open high end), the P - 2
-// middle ones (both ends open, equal lengths) and the last.  One launch
-// solves every piece with its halo read from the neighbouring pieces and
-// writes its heads and tails; a second forms the reduced system's unknowns
-// beside each piece from the dense inverse G and corrects:
-// x = y - V z_prev - W z_next.
-constexpr int kSigFields = 12;   // fields per pass (larger counts run in passes)
-struct SigPlan {
-    int P = 0, q = 1;
-    int len[3] = {0, 0, 0};        // piece length of the first, middle and last class
-    int64_t lines = 0;             // lines of the whole plan
-    CompactPlan cls[3];            // local plans of the classes (forced equal S and LB)
-    int dtype = CLES_F64;
-    void* tab = nullptr;           // class c: V [q][len_c], W [q][len_c]; then G (2qP)^2; plan dtype
-    int64_t off_V[3] = {0, 0, 0}, off_W[3] = {0, 0, 0}, off_G = 0;
-    void* loc = nullptr;           // local solutions: kSigFields x lines x n
-    void* iface[3] = {nullptr, nullptr, nullptr};   // heads / tails: kSigFields x 2q x lines of the class
-    ~SigPlan();
 };
 
 // Builds the plan of `scheme` along `dim` (0-based) of a grid with interior
@@ -173,12 +187,9 @@ struct SigPlan {
 // lo_open / hi_open make that end of a non-periodic line a rank interface.
 // pow2_seg_max > 0 (batched plans): S is the fewest power-of-two segments of
 // at most pow2_seg_max (8, 16 or 32) points.
-// force_S / force_LB > 0 fix the segments per line and the lines per CTA (the
-// classes of a SigPlan, which share one launch).
 void build_compact_plan(CompactPlan& plan, const cles_scheme& scheme, const int n3[3], int dim,
                         bool periodic, double h, int dtype, int lo_fold = 0, int hi_fold = 0,
-                        bool lo_open = false, bool hi_open = false, int pow2_seg_max = 0, int force_S = 0,
-                        int force_LB = 0);
+                        bool lo_open = false, bool hi_open = false, int pow2_seg_max = 0);
 
 // The LHS band of one line (or one rank's piece of a split line), row-major
 // n x (2q+1): interior band, closure rows at closed ends, parity folds, and
@@ -206,6 +217,7 @@ struct RkEpilogue {
     const double* dtp;  // when set, dt is read from device memory (graph mode)
 };
 
+int num_sms();   // multiprocessors of the current device
 // TMA-pipelined y/z launch; false when the plan or the views do not qualify.
 bool try_launch_tma(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
                     cudaStream_t st, const RkEpilogue* rk = nullptr);
@@ -213,10 +225,16 @@ bool try_launch_tma(const CompactPlan& plan, const FieldView& in, const FieldVie
 // staging into a transposed shared-memory tile; false if the plan does not fit.
 bool try_launch_xt(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
                    cudaStream_t st);
+// k_line launch; false (and nothing launched) when the plan has no line form.
+// rk: the RK update of mode OUT_RK; rk_first: no earlier direction stored into
+// `out`, the divergence is this direction's alone.
+bool try_launch_line(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
+                     cudaStream_t st, const RkEpilogue* rk = nullptr, bool rk_first = false);
 // Flux divergence of the last direction fused with the RK update; false (and
-// nothing launched) when the plan does not take the TMA path.
+// nothing launched) when the plan takes neither the TMA path nor k_line.  first:
+// the only direction, `out` holds nothing yet (and is not written).
 bool launch_compact_rk(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count,
-                       const RkEpilogue& rk, cudaStream_t st);
+                       const RkEpilogue& rk, cudaStream_t st, bool first = false);
 // One rank's piece of a line split across `ranks` ranks along `dim`
 // (src/decomposition.jl:73-78 local_range; src/tridiag.jl:85-170 and
 // src/banded.jl:108-214 with P > 1).  `local` solves the rank's own rows with

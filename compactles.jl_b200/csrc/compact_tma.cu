@@ -844,6 +844,7 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 int g_num_sms = 0;
+}  // namespace
 
 int num_sms() {
     if (!g_num_sms) {
@@ -853,6 +854,8 @@ int num_sms() {
     }
     return g_num_sms;
 }
+
+namespace {
 
 // Tiles in flight (1 to 3) for a CTA that shares its SM with another: half of
 // the 227 KB, less 1 KB the runtime reserves per CTA and the CTA's own
@@ -1144,21 +1147,6 @@ bool try_launch_tg_split(const CompactPlan& plan, const FieldView& in, const Fie
     if (plan.dtype == CLES_F64)
         return launch_tg<double>(plan, map, out, count, OUT_STORE, st, plan.tab64, rk, H, static_cast<double*>(iface));
     return launch_tg<float>(plan, map, out, count, OUT_STORE, st, plan.tab32, rk, H, static_cast<float*>(iface));
-}
-
-bool launch_compact_rk(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count,
-                       const RkEpilogue& rk, cudaStream_t st) {
-    if (count <= 0 || plan.P.lines == 0) return false;
-    int rec = -1;
-    if (profiling()) {
-        const double el = plan.dtype == CLES_F64 ? 8.0 : 4.0;
-        const double pts = (double)plan.P.lines * plan.P.n * count;
-        // input read, dQ read, du and Q read and written (8 bytes each)
-        rec = prof_begin(st, plan.P.dim, pts * (2.0 * el + 32.0));
-    }
-    const bool ok = try_launch_tma(plan, in, out, count, OUT_RK, st, &rk);
-    if (rec >= 0) prof_end(rec, st);
-    return ok;
 }
 
 // The expiry path of the bounded wait, run on purpose: one CTA initialises an

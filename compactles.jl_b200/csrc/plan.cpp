@@ -202,7 +202,279 @@ void build_warp_line(CompactPlan& plan, const Band& B, const cles_scheme& s, int
     plan.has_xw = true;
 }
 
+// ---- line form of any length (k_line) --------------------------------------
+
+template <typename T, int Q, int MS>
+void pack_line_coef(LinePlan& lp, const CompactParams& P, const std::vector<double> f[4][5], const std::vector<double> v[4][2],
+                    const std::vector<double> w[4][2], const double tl[4][4]) {
+    lp.coef.assign(sizeof(LineCoef<T, Q, MS>), 0);
+    auto* C = reinterpret_cast<LineCoef<T, Q, MS>*>(lp.coef.data());
+    for (int c = 0; c < 4; ++c) {
+        for (int a = 0; a < (Q == 1 ? 3 : 5); ++a)
+            for (int i = 0; i < MS; ++i) C->f[c][a][i] = T(f[c][a][i]);
+        for (int t = 0; t < Q; ++t)
+            for (int i = 0; i < MS; ++i) {
+                C->v[c][t][i] = T(v[c][t][i]);
+                C->w[c][t][i] = T(w[c][t][i]);
+            }
+        for (int e = 0; e < 4; ++e) C->tl[c][e] = T(tl[c][e]);
+    }
+    for (int i = 0; i < kMaxClo; ++i)
+        for (int k = 0; k < kMaxCloLen; ++k) {
+            C->clo[i][k] = T(P.clo[i][k]);
+            C->chi[i][k] = T(P.chi[i][k]);
+        }
+    for (int k = 0; k < CLES_MAX_M; ++k) C->ci[k] = T(P.ci[k]);
+    C->a0 = T(P.a0);
+}
+
+template <typename T, int Q>
+void pack_line_coef(LinePlan& lp, const CompactParams& P, const std::vector<double> f[4][5], const std::vector<double> v[4][2],
+                    const std::vector<double> w[4][2], const double tl[4][4]) {
+    if (lp.MS == 16) pack_line_coef<T, Q, 16>(lp, P, f, v, w, tl);
+    else if (lp.MS == 24) pack_line_coef<T, Q, 24>(lp, P, f, v, w, tl);
+    else pack_line_coef<T, Q, 32>(lp, P, f, v, w, tl);
+}
+
+// Segments of at most MS points: 32 per thread where the plan's points fill
+// the device with them, 16 below that (twice the threads, half the chain).
+constexpr int64_t kLineWide = (int64_t)1 << 21;
+
+void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
+    const CompactParams& P = plan.P;
+    const int n = P.n, q = P.q;
+    const bool periodic = B.periodic;
+    if (!((q == 1 && (P.M == 1 || P.M == 2 || P.M == 4)) || (q == 2 && P.M == 3))) return;
+    auto lp = std::unique_ptr<LinePlan>(new LinePlan());
+    const bool wide = P.lines * n >= kLineWide && n > 32;
+    int S = (n + (wide ? 31 : 15)) / (wide ? 32 : 16);
+    // Short-tile x plans run few lines a block, whose neighbouring threads read
+    // shared rows a segment length apart: an odd length keeps them on different
+    // banks.
+    if (P.dim == 0 && !wide)
+        for (int s = S; s <= S + S / 4 + 1; ++s) {
+            const int b = n / s, major = n % s > s / 2 ? b + 1 : b;
+            if (major & 1) { S = s; break; }
+        }
+    // two segments at least, long enough for the end rows, the stencil and the
+    // closure rows' reads to stay within a segment and its halo
+    if (S < 2 || S > 512 || n / S < 9) return;   // base >= 9 > 16 - 8, see ln_group
+    lp->S = S;
+    lp->base = n / S;
+    lp->rem = n % S;
+    lp->mm = (lp->base + (lp->rem ? 1 : 0) + 3) / 4 * 4;
+    const int MS = lp->mm <= 16 ? 16 : lp->mm <= 24 ? 24 : 32;
+    lp->MS = MS;
+    for (int j = 0; j < P.nc; ++j)
+        if (P.clo_len[j] > lp->base || P.clo_len[j] > kMaxCloLen) return;
+    auto off = [&](int s) { return s * lp->base + std::min(s, lp->rem); };
+    auto len = [&](int s) { return lp->base + (s < lp->rem ? 1 : 0); };
+    auto kind = [&](int s) { return !periodic && s == 0 ? 0 : !periodic && s == S - 1 ? 3 : s < lp->rem ? 1 : 2; };
+    std::vector<double> f[4][5], v[4][2], w[4][2];
+    std::vector<double> V[4][2], W[4][2];   // spikes at their own length
+    double tl[4][4] = {};
+    int have[4] = {0, 0, 0, 0};
+    for (int c = 0; c < 4; ++c) {
+        for (auto& a : f[c]) a.assign(MS, 0.0);
+        for (int t = 0; t < 2; ++t) {
+            v[c][t].assign(MS, 0.0);
+            w[c][t].assign(MS, 0.0);
+        }
+    }
+    for (int s = 0; s < S; ++s) {
+        const int c = kind(s);
+        if (have[c]) continue;
+        have[c] = 1;
+        const int o = off(s), m = len(s);
+        LocalFactor F;
+        F.build(B, o, m);
+        for (int i = 0; i < m; ++i) {
+            const double u0 = 1.0 / F.U[i];
+            const double u1 = i < m - 1 ? F.U[(size_t)m + i] * u0 : 0.0;
+            if (q == 1) {
+                f[c][0][i] = i > 0 ? F.L[(size_t)i - 1] : 0.0;
+                f[c][1][i] = u0;
+                f[c][2][i] = u1;
+            } else {
+                f[c][0][i] = i < m - 1 ? F.L[i] : 0.0;
+                f[c][1][i] = i < m - 2 ? F.L[(size_t)m + i] : -1.0;
+                f[c][2][i] = u1;
+                f[c][3][i] = i < m - 2 ? F.U[(size_t)2 * m + i] * u0 : 0.0;
+                f[c][4][i] = u0;
+            }
+        }
+        for (int i = m; i < MS; ++i) f[c][q == 1 ? 0 : 1][i] = -1.0;
+        tl[c][0] = 1.0 / F.U[(size_t)m - 1];
+        if (q == 2) {
+            tl[c][1] = F.U[(size_t)m + m - 2] / F.U[(size_t)m - 2];
+            tl[c][2] = 1.0 / F.U[(size_t)m - 2];
+            tl[c][3] = (lp->mm - m) & 1;
+        }
+        for (int t = 0; t < q; ++t) {
+            V[c][t].assign(m, 0.0);
+            W[c][t].assign(m, 0.0);
+            const bool prev = periodic || s > 0, next = periodic || s < S - 1;
+            if (prev) {
+                const int col = ((o - q + t) % n + n) % n;
+                for (int r = 0; r < q; ++r) V[c][t][r] = B.at(o + r, col);
+                F.solve(V[c][t].data());
+            }
+            if (next) {
+                const int col = (o + m + t) % n;
+                for (int r = m - q; r < m; ++r) W[c][t][r] = B.at(o + r, col);
+                F.solve(W[c][t].data());
+            }
+            for (int i = 0; i < m; ++i) {
+                v[c][t][i] = V[c][t][i];
+                w[c][t][i] = W[c][t][i];
+            }
+        }
+    }
+    if (dtype == CLES_F64) {
+        if (q == 1) pack_line_coef<double, 1>(*lp, P, f, v, w, tl);
+        else pack_line_coef<double, 2>(*lp, P, f, v, w, tl);
+    } else {
+        if (q == 1) pack_line_coef<float, 1>(*lp, P, f, v, w, tl);
+        else pack_line_coef<float, 2>(*lp, P, f, v, w, tl);
+    }
+
+    // Rows of the inverse of the reduced system in z = (head_0, tail_0, ...) for
+    // the unknowns of segment s, from the chain of segments [s - K, s + K] (all
+    // of the line where that covers it).  The chain's cut ends must not matter:
+    // K doubles until what the rows hold in their outermost segments is below
+    // the threshold.  Rows depend on the kinds of the chain's segments only.
+    const double thr = dtype == CLES_F64 ? std::ldexp(1.0, -60) : std::ldexp(1.0, -34);
+    const int b2 = 2 * q;
+    struct Rows {
+        int first = 0, nseg = 0;     // relative to s; segments held
+        std::vector<double> g;       // [2q][nseg][2q]
+    };
+    auto inverse_rows = [&](int s, int K, bool whole) {
+        const int lo = whole ? (periodic ? s : 0) : periodic ? s - K : std::max(0, s - K);
+        const int hi = whole ? (periodic ? s + S - 1 : S - 1) : periodic ? s + K : std::min(S - 1, s + K);
+        const int ns = hi - lo + 1, N = b2 * ns;
+        std::vector<double> R((size_t)N * N, 0.0);
+        for (int a = 0; a < ns; ++a) {
+            const int c = kind((((lo + a) % S) + S) % S), m = (int)V[c][0].size();
+            const int pa = whole && periodic ? (a - 1 + ns) % ns : a - 1;
+            const int na = whole && periodic ? (a + 1) % ns : (a + 1 < ns ? a + 1 : -1);
+            for (int r = 0; r < q; ++r) {
+                const size_t rh = (size_t)(b2 * a + r) * N, rt = (size_t)(b2 * a + q + r) * N;
+                R[rh + b2 * a + r] += 1.0;
+                R[rt + b2 * a + q + r] += 1.0;
+                for (int t = 0; t < q; ++t) {
+                    if (pa >= 0) {
+                        R[rh + b2 * pa + q + t] += V[c][t][r];
+                        R[rt + b2 * pa + q + t] += V[c][t][m - q + r];
+                    }
+                    if (na >= 0) {
+                        R[rh + b2 * na + t] += W[c][t][r];
+                        R[rt + b2 * na + t] += W[c][t][m - q + r];
+                    }
+                }
+            }
+        }
+        const std::vector<double> G = dense_inverse(R, N);
+        Rows out;
+        out.first = lo - s;
+        out.nseg = ns;
+        out.g.resize((size_t)b2 * N);
+        for (int r = 0; r < b2; ++r)
+            for (int j = 0; j < N; ++j) out.g[(size_t)r * N + j] = G[(size_t)(b2 * (s - lo) + r) * N + j];
+        return out;
+    };
+    std::vector<int> row_of(S);
+    std::vector<Rows> rows;
+    int Kr = 0;
+    for (int K = 4;; K *= 2) {
+        const bool whole = 2 * K + 1 >= S;
+        rows.clear();
+        Kr = 0;
+        bool good = true;
+        std::vector<std::pair<std::vector<int>, int>> seen;   // chain pattern -> rows entry
+        for (int s = 0; s < S && good; ++s) {
+            std::vector<int> pat;
+            if (whole) pat.push_back(s);
+            else
+                for (int a = s - K; a <= s + K; ++a) {
+                    if (!periodic && (a < 0 || a >= S)) pat.push_back(-1);
+                    else pat.push_back(kind(((a % S) + S) % S));
+                }
+            int e = -1;
+            for (const auto& pr : seen)
+                if (pr.first == pat) { e = pr.second; break; }
+            if (e < 0) {
+                e = (int)rows.size();
+                rows.push_back(inverse_rows(s, K, whole));
+                seen.emplace_back(pat, e);
+                const Rows& R = rows.back();
+                for (int r = 0; r < b2; ++r) {
+                    // weight of the row's entries by their distance from s
+                    std::vector<double> wt((size_t)(whole ? S : K) + 1, 0.0);
+                    double sum = 0.0;
+                    for (int a = 0; a < R.nseg; ++a) {
+                        int d = std::abs(R.first + a);
+                        if (whole && periodic) d = std::min(d, S - d);
+                        for (int u = 0; u < b2; ++u) {
+                            const double x = std::fabs(R.g[(size_t)r * b2 * R.nseg + b2 * a + u]);
+                            wt[d] += x;
+                            sum += x;
+                        }
+                    }
+                    int k = (int)wt.size() - 1;
+                    double tail = 0.0;
+                    while (k > 0 && tail + wt[k] <= thr * sum) tail += wt[k--];
+                    Kr = std::max(Kr, k);
+                    if (!whole && k >= K) good = false;
+                }
+            }
+            row_of[s] = e;
+        }
+        if (good || whole) break;
+    }
+    const int Wn = std::min(2 * Kr + 1, S);
+    if (Wn * b2 > 96) return;   // slowly decaying scheme: the dense or cyclic forms serve it better
+    lp->Wn = Wn;
+    lp->Kr = Kr;
+    std::vector<double> tab((size_t)S * b2 * Wn * b2, 0.0);
+    for (int s = 0; s < S; ++s)
+        for (int side = 0; side < 2; ++side) {
+            const int raw = side == 0 ? s - 1 : s + 1;
+            if (!periodic && (raw < 0 || raw >= S)) continue;
+            const int rs = (raw + S) % S;
+            const Rows& R = rows[row_of[rs]];
+            const int start = periodic ? raw - Kr : std::max(0, std::min(raw - Kr, S - Wn));
+            for (int t = 0; t < q; ++t) {
+                const int r = side == 0 ? q + t : t;   // the previous tails, the next heads
+                for (int j = 0; j < Wn; ++j) {
+                    int a = start + j - raw - R.first;   // segment within the rows
+                    if (periodic && R.nseg == S) a = ((a % S) + S) % S;
+                    if (a < 0 || a >= R.nseg) continue;
+                    for (int u = 0; u < b2; ++u)
+                        tab[(((size_t)s * b2 + side * q + t) * Wn + j) * b2 + u] =
+                            R.g[(size_t)r * b2 * R.nseg + b2 * a + u];
+                }
+            }
+        }
+    if (dtype == CLES_F64) {
+        CLES_CUDA(cudaMalloc(&lp->tab, sizeof(double) * tab.size()));
+        CLES_CUDA(cudaMemcpy(lp->tab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
+    } else {
+        std::vector<float> t32(tab.begin(), tab.end());
+        CLES_CUDA(cudaMalloc(&lp->tab, sizeof(float) * t32.size()));
+        CLES_CUDA(cudaMemcpy(lp->tab, t32.data(), sizeof(float) * t32.size(), cudaMemcpyHostToDevice));
+    }
+    CLES_CUDA(cudaMalloc(&lp->dcoef, lp->coef.size()));
+    CLES_CUDA(cudaMemcpy(lp->dcoef, lp->coef.data(), lp->coef.size(), cudaMemcpyHostToDevice));
+    plan.line = std::move(lp);
+}
+
 }  // namespace
+
+LinePlan::~LinePlan() {
+    if (tab) cudaFree(tab);
+    if (dcoef) cudaFree(dcoef);
+}
 
 CompactPlan::~CompactPlan() {
     if (tab64) cudaFree(tab64);
@@ -289,115 +561,8 @@ void LineBand::solve(double* x) const {
     }
 }
 
-// The pieces of a SigPlan: P = ceil(n / 128) (at most 64) pieces, the middle
-// ones of equal length n / P and the remainder shared by the first and last;
-// S segments of at most 16 points in every piece (32 beyond 512-point
-// pieces), two pieces per CTA.  Spikes of each class and the reduced system
-// over all pieces as in build_split_plan (the rank-level spikes of
-// src/tridiag.jl:85-123 and src/banded.jl:108-169), its dense inverse whole.
-static void build_sig_plan(CompactPlan& plan, const cles_scheme& s, const int n3[3], double h, int dtype) {
-    const int n = n3[0], q = s.q;
-    const int P = std::min(64, (n + 127) / 128);
-    if (P < 4) return;
-    // pieces of at most 1024 points (the correction's four points a thread)
-    if ((n / P) + (n % P) > 1024) return;
-    const int mid = n / P, rem = n - P * mid;
-    const int len[3] = {mid + rem / 2, mid, mid + (rem - rem / 2)};
-    const int maxlen = std::max(len[0], len[2]);
-    int S = (maxlen + 15) / 16;
-    if (S > 32) S = (maxlen + kMaxSeg - 1) / kMaxSeg;
-    if (S > 32 || mid / S < std::max(2 * q + 1, q + 1)) return;
-    const int LB = 2;
-    auto sp = std::unique_ptr<SigPlan>(new SigPlan());
-    sp->P = P;
-    sp->q = q;
-    sp->lines = plan.P.lines;
-    sp->dtype = dtype;
-    for (int c = 0; c < 3; ++c) sp->len[c] = len[c];
-    const int L = (int)plan.P.lines;
-    for (int c = 0; c < 3; ++c) {
-        // the middle class enumerates (piece - 1) fastest, then the line
-        int nc3[3] = {len[c], c == 1 ? P - 2 : L, c == 1 ? L : 1};
-        build_compact_plan(sp->cls[c], s, nc3, 0, false, h, dtype, 0, 0, c > 0, c < 2, 0, S, LB);
-        if (sp->cls[c].P.pcr || sp->cls[c].P.S != S || sp->cls[c].P.LB != LB) return;
-    }
-    // spikes per class, reduced system in z = (head_0, tail_0, head_1, ...)
-    std::vector<double> Vc[3], Wc[3];
-    for (int c = 0; c < 3; ++c) {
-        const int m = len[c];
-        const bool lo = c > 0, hi = c < 2;
-        LineBand b = make_line_band(s, m, 0, 0, lo, hi);
-        b.factor();
-        Vc[c].assign((size_t)q * m, 0.0);
-        Wc[c].assign((size_t)q * m, 0.0);
-        for (int t = 0; t < q; ++t) {
-            double* v = &Vc[c][(size_t)t * m];
-            double* w = &Wc[c][(size_t)t * m];
-            if (lo) {
-                for (int r = 0; r < q; ++r) {
-                    const int d = r + q - t;
-                    if (d >= 1 && d <= q) v[r] = s.lhs[d - 1];
-                }
-                b.solve(v);
-            }
-            if (hi) {
-                for (int i = m - q; i < m; ++i) {
-                    const int d = m + t - i;
-                    if (d >= 1 && d <= q) w[i] = s.lhs[d - 1];
-                }
-                b.solve(w);
-            }
-        }
-    }
-    const int N = 2 * q * P;
-    std::vector<double> R((size_t)N * N, 0.0);
-    for (int rr = 0; rr < P; ++rr) {
-        const int c = rr == 0 ? 0 : (rr == P - 1 ? 2 : 1), m = len[c];
-        for (int r = 0; r < q; ++r) {
-            const int rh = 2 * q * rr + r, rt = 2 * q * rr + q + r;
-            R[(size_t)rh * N + rh] += 1.0;
-            R[(size_t)rt * N + rt] += 1.0;
-            for (int t = 0; t < q; ++t) {
-                if (rr > 0) {
-                    const int cprev = 2 * q * (rr - 1) + q + t;
-                    R[(size_t)rh * N + cprev] += Vc[c][(size_t)t * m + r];
-                    R[(size_t)rt * N + cprev] += Vc[c][(size_t)t * m + (m - q + r)];
-                }
-                if (rr < P - 1) {
-                    const int cnext = 2 * q * (rr + 1) + t;
-                    R[(size_t)rh * N + cnext] += Wc[c][(size_t)t * m + r];
-                    R[(size_t)rt * N + cnext] += Wc[c][(size_t)t * m + (m - q + r)];
-                }
-            }
-        }
-    }
-    const std::vector<double> G = dense_inverse(R, N);
-    std::vector<double> tab;
-    for (int c = 0; c < 3; ++c) {
-        sp->off_V[c] = (int64_t)tab.size();
-        tab.insert(tab.end(), Vc[c].begin(), Vc[c].end());
-        sp->off_W[c] = (int64_t)tab.size();
-        tab.insert(tab.end(), Wc[c].begin(), Wc[c].end());
-    }
-    sp->off_G = (int64_t)tab.size();
-    tab.insert(tab.end(), G.begin(), G.end());
-    const size_t el = dtype == CLES_F64 ? sizeof(double) : sizeof(float);
-    CLES_CUDA(cudaMalloc(&sp->tab, el * tab.size()));
-    if (dtype == CLES_F64) {
-        CLES_CUDA(cudaMemcpy(sp->tab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
-    } else {
-        std::vector<float> t32(tab.begin(), tab.end());
-        CLES_CUDA(cudaMemcpy(sp->tab, t32.data(), sizeof(float) * t32.size(), cudaMemcpyHostToDevice));
-    }
-    CLES_CUDA(cudaMalloc(&sp->loc, el * (size_t)kSigFields * (size_t)L * (size_t)n));
-    for (int c = 0; c < 3; ++c)
-        CLES_CUDA(cudaMalloc(&sp->iface[c], el * (size_t)kSigFields * 2 * q * (size_t)sp->cls[c].P.lines));
-    plan.sig = std::move(sp);
-}
-
 void build_compact_plan(CompactPlan& plan, const cles_scheme& s, const int n3[3], int dim, bool periodic,
-                        double h, int dtype, int lo_fold, int hi_fold, bool lo_open, bool hi_open, int pow2_seg_max,
-                        int force_S, int force_LB) {
+                        double h, int dtype, int lo_fold, int hi_fold, bool lo_open, bool hi_open, int pow2_seg_max) {
     const int n = n3[dim];
     const int q = s.q, M = s.M, nc = s.nc;
     if (q < 1 || q > CLES_MAX_Q) throw Error(CLES_EINVAL, "scheme LHS half-bandwidth q must be 1 or 2");
@@ -528,10 +693,6 @@ void build_compact_plan(CompactPlan& plan, const cles_scheme& s, const int n3[3]
         while ((n + S - 1) / S > std::min(pow2_seg_max, kMaxSeg)) S *= 2;
         if (n / S < std::max(2 * q + 1, q + 1)) throw Error(CLES_EINVAL, "batched segments too short for the scheme");
     }
-    if (force_S > 0) {
-        S = force_S;
-        if (n / S < std::max(2 * q + 1, q + 1)) throw Error(CLES_EINVAL, "forced segments too short for the scheme");
-    }
     P.S = S;
     P.seg_base = n / S;
     P.seg_rem = n % S;
@@ -547,10 +708,9 @@ void build_compact_plan(CompactPlan& plan, const cles_scheme& s, const int n3[3]
         while (LB > 1 && (size_t)n * (LB + 1) * el > 110 * 1024) LB /= 2;
         if ((size_t)n * (LB + 1) * el > 200 * 1024) throw Error(CLES_EINVAL, "x line too long for the shared-memory tile");
     }
-    if (force_LB > 0) LB = force_LB;
     if (LB * S > 512) throw Error(CLES_EINVAL, "line too long for one CTA");
     const int LB_full = LB;
-    if (P.lines < LB && force_LB <= 0) {
+    if (P.lines < LB) {
         int l = 1;
         while (l < P.lines) l *= 2;
         LB = std::max(1, std::min(LB, l));
@@ -777,18 +937,7 @@ void build_compact_plan(CompactPlan& plan, const cles_scheme& s, const int n3[3]
         CLES_CUDA(cudaMalloc(&plan.tab32, sizeof(float) * total));
         CLES_CUDA(cudaMemcpy(plan.tab32, t32.data(), sizeof(float) * total, cudaMemcpyHostToDevice));
     }
-    // a handful of long closed x lines is latency-bound in one CTA per line:
-    // cut it into pieces solved side by side (SigPlan)
-    if (dim == 0 && !periodic && !lo_fold && !hi_fold && !lo_open && !hi_open && pow2_seg_max == 0 &&
-        force_S == 0 && P.lines <= 16 && n >= 2048 && (n3[1] == 1 || n3[2] == 1))
-        build_sig_plan(plan, s, n3, h, dtype);
-}
-
-SigPlan::~SigPlan() {
-    if (tab) cudaFree(tab);
-    if (loc) cudaFree(loc);
-    for (void* p : iface)
-        if (p) cudaFree(p);
+    if (!lo_open && !hi_open && pow2_seg_max == 0) build_line_plan(plan, B, dtype);
 }
 
 SplitPlan::~SplitPlan() {

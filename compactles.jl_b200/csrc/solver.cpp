@@ -926,8 +926,8 @@ public:
             const FieldView fin = view(fk);
             if (split_[k].on) {
                 split_apply(*split_[k].deriv, k, fk, fk, dQ_.p, ncons_, first ? OUT_NEGATE : OUT_SUBTRACT);
-            } else if (k == last && !first && rk &&
-                       launch_compact_rk(*dset_[k][0], fin, view(dQ_.as<F>()), ncons_, *rk, st_)) {
+            } else if (k == last && rk &&
+                       launch_compact_rk(*dset_[k][0], fin, view(dQ_.as<F>()), ncons_, *rk, st_, first)) {
                 fused = true;
             } else {
                 launch_compact(*dset_[k][0], fin, view(dQ_.as<F>()), ncons_, first ? OUT_NEGATE : OUT_SUBTRACT, st_);
