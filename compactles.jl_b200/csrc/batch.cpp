@@ -11,7 +11,7 @@
 // reads.  Everything that depends on a grid's shape or spacing takes a table:
 //   * line solves: a launch table of per-grid plans (power-of-two segments)
 //     and a CTA table (launch_compact_batch);
-//   * delta4_sum!: a table of 32 x 16 x 32 tiles;
+//   * delta4_sum!: a table of 32 x 16 x 16 tiles;
 //   * boundary planes: a table of faces;
 //   * max_rate + the graph-mode clock: a table of 2048-cell chunks, then one
 //     block per grid; every grid keeps its own dt, clock and stop condition.
@@ -527,7 +527,7 @@ private:
         prim_.alloc(ctx_, Fs * c * (P_Y0 + Ns_ + 1));
         g_u_.alloc(ctx_, Fs * c * 9);
         gty_.alloc(ctx_, Fs * c * 3 * (1 + Ns_));
-        scratch_.alloc(ctx_, Fs * c * 5);
+        scratch_.alloc(ctx_, Fs * c * std::max(5, 3 + Ns_));
         flux_.alloc(ctx_, Fs * c * 3 * ncons_);
         for (DevBuf* b : {&du_, &dQ_, &prim_, &g_u_, &gty_, &scratch_, &flux_})
             CLES_CUDA(cudaMemsetAsync(b->p, 0, b->bytes, st_));
@@ -822,8 +822,8 @@ private:
     void bcs() {
         batch_bc(Q_.as<double>(), grids_.as<BatchGrid>(), faces_.as<BatchFace>(), nfaces_, ct_, Ns_, st_);
     }
-    void delta4(const F* f0, const F* f1, F* o0, F* o1, int p0, int p1) {
-        BatchOps<F>::delta4(f0, f1, o0, o1, p0, p1, grids_.as<BatchGrid>(), tiles_.as<BatchTile>(), ntiles_, ct_, st_);
+    void delta4(const D4Set<F>& fs) {
+        BatchOps<F>::delta4(fs, grids_.as<BatchGrid>(), tiles_.as<BatchTile>(), ntiles_, st_);
     }
 
     void artificial() {
@@ -832,27 +832,26 @@ private:
         if (!cls_.art_enabled) return;
         using PW = Pointwise<F>;
         F* strain = field(scratch_, 0);
-        F* sensor = field(scratch_, 1);
-        F* sensor_e = field(scratch_, 2);
-        F* tmp_a = field(scratch_, 3);
-        F* tmp_b = field(scratch_, 4);
-        PW::strain(g_u_.as<F>(), strain, ct_, st_);
-        delta4(strain, field(prim_, P_Y0 + Ns_), sensor, sensor_e, 2, 1);
-        smooth(sensor, 2);
-        PW::art_coef(sensor, sensor_e, prim_.as<F>(), g_u_.as<F>(), art_.as<F>(), ct_, cls_.C_mu, cls_.C_beta,
-                     cls_.C_kappa, cls_.beta_sensor == CLES_BETA_GATED_STRAIN, st_);
+        F* sensors = field(scratch_, 1);
+        const int ns = Ns_ > 1 ? 2 + Ns_ : 2;
+        PW::strain(g_u_.as<F>(), strain, ct_, dims(), st_);
+        D4Set<F> fs;
+        fs.add(strain, sensors, 2);
+        fs.add(field(prim_, P_Y0 + Ns_), field(scratch_, 2), 1);
+        for (int sp = 0; sp < ns - 2; ++sp) fs.add(field(prim_, P_Y0 + sp), field(scratch_, 3 + sp), 1);
+        delta4(fs);
+        smooth(sensors, ns);
+        PW::art_coef(sensors, prim_.as<F>(), g_u_.as<F>(), art_.as<F>(), ct_, Ns_, cls_.C_mu, cls_.C_beta, cls_.C_kappa,
+                     cls_.C_D, cls_.beta_sensor == CLES_BETA_GATED_STRAIN, st_);
         if (cls_.beta_sensor == CLES_BETA_DILATATION) {
+            F* tmp_a = field(scratch_, 3);
+            F* tmp_b = field(scratch_, 4);
             PW::dilatation(g_u_.as<F>(), tmp_a, tmp_b, ct_, st_);
-            delta4(tmp_a, nullptr, sensor, nullptr, 2, 2);
-            smooth(sensor, 1);
-            PW::beta_dilatation(sensor, prim_.as<F>(), tmp_b, art_.as<F>(), ct_, cls_.C_beta, st_);
-        }
-        if (Ns_ > 1) {
-            for (int sp = 0; sp < Ns_; ++sp) {
-                delta4(field(prim_, P_Y0 + sp), nullptr, tmp_a, nullptr, 1, 1);
-                smooth(tmp_a, 1);
-                PW::dart(tmp_a, prim_.as<F>(), art_.as<F>(), ct_, cls_.C_D, sp, st_);
-            }
+            D4Set<F> fd;
+            fd.add(tmp_a, sensors, 2);
+            delta4(fd);
+            smooth(sensors, 1);
+            PW::beta_dilatation(sensors, prim_.as<F>(), tmp_b, art_.as<F>(), ct_, cls_.C_beta, st_);
         }
     }
 
@@ -866,7 +865,7 @@ private:
         for (int k = 0; k < 3; ++k)
             if (act_[k]) along(R_DERIV, k, field(prim_, P_T), gty_.as<F>() + (size_t)ct_ * ngty * k, ngty, OUT_STORE);
         BatchOps<F>::fluxes(Q_.as<double>(), prim_.as<F>(), g_u_.as<F>(), gty_.as<F>(), art_.as<F>(), flux_.as<F>(),
-                            ct_, Ns_, pc_, cls_.mu0, cls_.Pr, cls_.Sc, mc_.as<double>(), tmap_.as<int>(), st_);
+                            ct_, Ns_, pc_, cls_.mu0, cls_.Pr, cls_.Sc, dims(), mc_.as<double>(), tmap_.as<int>(), st_);
         // dQ = -sum_d D_d(F_d) with the RK update in the last direction's store
         // (y, x, z on 3-D grids, as the solver orders them)
         int order[3] = {0, 1, 2};
@@ -888,6 +887,7 @@ private:
             BatchOps<F>::lsrk(Q_.as<double>(), du_.as<double>(), dQ_.as<F>(), ct_, ncons_, tmap_.as<int>(),
                               grids_.as<BatchGrid>(), need_lsrk_.as<int>(), kLsrkA[stage], kLsrkB[stage], st_);
     }
+    int dims() const { return (act_[0] ? 1 : 0) | (act_[1] ? 2 : 0) | (act_[2] ? 4 : 0); }
     int last_dim() const {
         int l = 0;
         for (int k = 0; k < 3; ++k)

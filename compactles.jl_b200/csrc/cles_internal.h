@@ -146,9 +146,9 @@ struct LinePlan {
     int mm = 0;                       // longest segment, rounded up to a group of four rows
     int Wn = 0, Kr = 0;               // interface window: segments, radius
     std::vector<unsigned char> coef;  // LineCoef<plan dtype, q, MS>
-    void* dcoef = nullptr;            // the same on the device
-    void* tab = nullptr;              // reduced inverse rows, [S][2q][Wn][2q], plan dtype
-    ~LinePlan();
+    std::vector<unsigned char> host_tab;   // reduced inverse rows, [S][2q][Wn][2q], until they are on the device
+    const void* dcoef = nullptr;      // coef and those rows in the plan's device block
+    const void* tab = nullptr;
 };
 struct LineArgs {
     FieldView in, out;
@@ -173,7 +173,8 @@ struct CompactPlan {
     WarpLineParams XW;
     CompactParams P;
     int dtype = CLES_F64;
-    double* tab64 = nullptr;
+    void* dev = nullptr;     // device block of all tables
+    double* tab64 = nullptr; // into dev
     float* tab32 = nullptr;
     size_t tab_elems = 0;
     std::unique_ptr<LinePlan> line;   // k_line form, where the plan has one

@@ -296,7 +296,7 @@ void MetricOps<F>::rate_geo(const double* Q, const F* prim, const F* art, double
                             const double h[3], double mu0, double Pr, double Sc, const Geom& G, const Grid3& gr,
                             cudaStream_t st) {
     const int64_t cells = (int64_t)gr.n[0] * gr.n[1] * gr.n[2];
-    const unsigned nb = grid_for(cells);
+    const unsigned nb = (unsigned)rate_partials(cells);
     k_rate_partial_geo<F><<<nb, kThreads, 0, st>>>(Q, prim, art, part, Ns, h[0], h[1], h[2], mu0, Pr, Sc, G, gr,
                                                    cells);
     count_launch();

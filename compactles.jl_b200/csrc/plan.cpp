@@ -349,38 +349,75 @@ void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
         int first = 0, nseg = 0;     // relative to s; segments held
         std::vector<double> g;       // [2q][nseg][2q]
     };
-    auto inverse_rows = [&](int s, int K, bool whole) {
-        const int lo = whole ? (periodic ? s : 0) : periodic ? s - K : std::max(0, s - K);
-        const int hi = whole ? (periodic ? s + S - 1 : S - 1) : periodic ? s + K : std::min(S - 1, s + K);
-        const int ns = hi - lo + 1, N = b2 * ns;
-        std::vector<double> R((size_t)N * N, 0.0);
+    // the reduced matrix of segments lo .. lo + ns - 1 (mod S), cyclic or cut
+    auto reduced = [&](int lo, int ns, bool cyclic, auto&& add) {
         for (int a = 0; a < ns; ++a) {
             const int c = kind((((lo + a) % S) + S) % S), m = (int)V[c][0].size();
-            const int pa = whole && periodic ? (a - 1 + ns) % ns : a - 1;
-            const int na = whole && periodic ? (a + 1) % ns : (a + 1 < ns ? a + 1 : -1);
+            const int pa = cyclic ? (a - 1 + ns) % ns : a - 1;
+            const int na = cyclic ? (a + 1) % ns : (a + 1 < ns ? a + 1 : -1);
             for (int r = 0; r < q; ++r) {
-                const size_t rh = (size_t)(b2 * a + r) * N, rt = (size_t)(b2 * a + q + r) * N;
-                R[rh + b2 * a + r] += 1.0;
-                R[rt + b2 * a + q + r] += 1.0;
+                const int rh = b2 * a + r, rt = b2 * a + q + r;
+                add(rh, rh, 1.0);
+                add(rt, rt, 1.0);
                 for (int t = 0; t < q; ++t) {
                     if (pa >= 0) {
-                        R[rh + b2 * pa + q + t] += V[c][t][r];
-                        R[rt + b2 * pa + q + t] += V[c][t][m - q + r];
+                        add(rh, b2 * pa + q + t, V[c][t][r]);
+                        add(rt, b2 * pa + q + t, V[c][t][m - q + r]);
                     }
                     if (na >= 0) {
-                        R[rh + b2 * na + t] += W[c][t][r];
-                        R[rt + b2 * na + t] += W[c][t][m - q + r];
+                        add(rh, b2 * na + t, W[c][t][r]);
+                        add(rt, b2 * na + t, W[c][t][m - q + r]);
                     }
                 }
             }
         }
-        const std::vector<double> G = dense_inverse(R, N);
+    };
+    std::vector<double> Gcyc;   // inverse of a whole periodic line
+    auto inverse_rows = [&](int s, int K, bool whole) {
         Rows out;
+        if (whole && periodic) {
+            const int N = b2 * S;
+            if (Gcyc.empty()) {
+                std::vector<double> R((size_t)N * N, 0.0);
+                reduced(0, S, true, [&](int i, int j, double x) { R[(size_t)i * N + j] += x; });
+                Gcyc = dense_inverse(R, N);
+            }
+            out.first = 0;   // segment s first
+            out.nseg = S;
+            out.g.resize((size_t)b2 * N);
+            for (int r = 0; r < b2; ++r)
+                for (int j = 0; j < N; ++j)
+                    out.g[(size_t)r * N + j] = Gcyc[(size_t)(b2 * s + r) * N + (j + b2 * s) % N];
+            return out;
+        }
+        // rows of the inverse of a chain: R^T x = e_r with the banded LU of R^T
+        // (half-bandwidth 3q - 1, unit diagonal plus the decayed spikes)
+        const int lo = whole ? 0 : periodic ? s - K : std::max(0, s - K);
+        const int hi = whole ? S - 1 : periodic ? s + K : std::min(S - 1, s + K);
+        const int ns = hi - lo + 1, N = b2 * ns, kb = 3 * q - 1, BW = 2 * kb + 1;
+        std::vector<double> A((size_t)N * BW, 0.0);
+        reduced(lo, ns, false, [&](int i, int j, double x) { A[(size_t)j * BW + kb + i - j] += x; });
+        for (int k = 0; k < N; ++k)
+            for (int i = k + 1; i <= std::min(N - 1, k + kb); ++i) {
+                const double l = A[(size_t)i * BW + kb + k - i] / A[(size_t)k * BW + kb];
+                A[(size_t)i * BW + kb + k - i] = l;
+                for (int j = k + 1; j <= std::min(N - 1, k + kb); ++j)
+                    A[(size_t)i * BW + kb + j - i] -= l * A[(size_t)k * BW + kb + j - k];
+            }
         out.first = lo - s;
         out.nseg = ns;
-        out.g.resize((size_t)b2 * N);
-        for (int r = 0; r < b2; ++r)
-            for (int j = 0; j < N; ++j) out.g[(size_t)r * N + j] = G[(size_t)(b2 * (s - lo) + r) * N + j];
+        out.g.assign((size_t)b2 * N, 0.0);
+        for (int r = 0; r < b2; ++r) {
+            double* x = &out.g[(size_t)r * N];
+            const int e = b2 * (s - lo) + r;
+            x[e] = 1.0;
+            for (int i = e + 1; i < N; ++i)
+                for (int k = std::max(e, i - kb); k < i; ++k) x[i] -= A[(size_t)i * BW + kb + k - i] * x[k];
+            for (int i = N - 1; i >= 0; --i) {
+                for (int k = i + 1; k <= std::min(N - 1, i + kb); ++k) x[i] -= A[(size_t)i * BW + kb + k - i] * x[k];
+                x[i] /= A[(size_t)i * BW + kb];
+            }
+        }
         return out;
     };
     std::vector<int> row_of(S);
@@ -456,29 +493,17 @@ void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
                 }
             }
         }
-    if (dtype == CLES_F64) {
-        CLES_CUDA(cudaMalloc(&lp->tab, sizeof(double) * tab.size()));
-        CLES_CUDA(cudaMemcpy(lp->tab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
-    } else {
-        std::vector<float> t32(tab.begin(), tab.end());
-        CLES_CUDA(cudaMalloc(&lp->tab, sizeof(float) * t32.size()));
-        CLES_CUDA(cudaMemcpy(lp->tab, t32.data(), sizeof(float) * t32.size(), cudaMemcpyHostToDevice));
-    }
-    CLES_CUDA(cudaMalloc(&lp->dcoef, lp->coef.size()));
-    CLES_CUDA(cudaMemcpy(lp->dcoef, lp->coef.data(), lp->coef.size(), cudaMemcpyHostToDevice));
+    const size_t el = dtype == CLES_F64 ? sizeof(double) : sizeof(float);
+    lp->host_tab.resize(el * tab.size());
+    if (dtype == CLES_F64) std::memcpy(lp->host_tab.data(), tab.data(), lp->host_tab.size());
+    else std::copy(tab.begin(), tab.end(), reinterpret_cast<float*>(lp->host_tab.data()));
     plan.line = std::move(lp);
 }
 
 }  // namespace
 
-LinePlan::~LinePlan() {
-    if (tab) cudaFree(tab);
-    if (dcoef) cudaFree(dcoef);
-}
-
 CompactPlan::~CompactPlan() {
-    if (tab64) cudaFree(tab64);
-    if (tab32) cudaFree(tab32);
+    if (dev) cudaFree(dev);
 }
 
 LineBand make_line_band(const cles_scheme& s, int n, int lo_fold, int hi_fold, bool lo_open, bool hi_open) {
@@ -930,14 +955,35 @@ void build_compact_plan(CompactPlan& plan, const cles_scheme& s, const int n3[3]
 
     plan.dtype = dtype;
     plan.tab_elems = (size_t)total;
-    CLES_CUDA(cudaMalloc(&plan.tab64, sizeof(double) * total));
-    CLES_CUDA(cudaMemcpy(plan.tab64, tab.data(), sizeof(double) * total, cudaMemcpyHostToDevice));
-    if (dtype == CLES_F32) {
-        std::vector<float> t32(tab.begin(), tab.end());
-        CLES_CUDA(cudaMalloc(&plan.tab32, sizeof(float) * total));
-        CLES_CUDA(cudaMemcpy(plan.tab32, t32.data(), sizeof(float) * total, cudaMemcpyHostToDevice));
-    }
     if (!lo_open && !hi_open && pow2_seg_max == 0) build_line_plan(plan, B, dtype);
+    // every table of the plan in one device block and one copy
+    std::vector<unsigned char> blob;
+    auto put = [&](const void* src, size_t bytes) {
+        const size_t at = (blob.size() + 255) / 256 * 256;
+        blob.resize(at + bytes);
+        std::memcpy(blob.data() + at, src, bytes);
+        return at;
+    };
+    const size_t at64 = put(tab.data(), sizeof(double) * tab.size());
+    size_t at32 = 0, at_lt = 0, at_lc = 0;
+    if (dtype == CLES_F32) {
+        const std::vector<float> t32(tab.begin(), tab.end());
+        at32 = put(t32.data(), sizeof(float) * t32.size());
+    }
+    if (plan.line) {
+        at_lt = put(plan.line->host_tab.data(), plan.line->host_tab.size());
+        at_lc = put(plan.line->coef.data(), plan.line->coef.size());
+        plan.line->host_tab = {};
+    }
+    CLES_CUDA(cudaMalloc(&plan.dev, blob.size()));
+    CLES_CUDA(cudaMemcpy(plan.dev, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+    auto* base_ptr = static_cast<unsigned char*>(plan.dev);
+    plan.tab64 = reinterpret_cast<double*>(base_ptr + at64);
+    if (dtype == CLES_F32) plan.tab32 = reinterpret_cast<float*>(base_ptr + at32);
+    if (plan.line) {
+        plan.line->tab = base_ptr + at_lt;
+        plan.line->dcoef = base_ptr + at_lc;
+    }
 }
 
 SplitPlan::~SplitPlan() {

@@ -7,6 +7,8 @@
 
 #include "pointwise.h"
 
+#include <algorithm>
+
 namespace cles {
 
 namespace {
@@ -91,67 +93,95 @@ inline unsigned grid_for(int64_t n) {
         check_launch(#kern);                                           \
     } while (0)
 
-// opt a kernel in to `bytes` of dynamic shared memory (above the 48 KB
-// default) on the current device; a host call, set before every launch so
-// that every device and thread sees it
-template <typename K>
-void set_smem_attr(K kern, size_t bytes) {
-    CLES_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+#define GRID_STRIDE(idx, n) for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < (n); idx += (int64_t)gridDim.x * blockDim.x)
+
+// Constants of the max_rate reduction (src/timestep.jl:125-175), Cartesian.
+struct RateConst {
+    double idx[3];   // 1 / h
+    int act[3];
+    double mu0, mu0_Pr, mu0_Sc;   // mu0, mu0 / Pr, mu0 / Sc
+};
+
+// The max_rate contribution of a cell from its primitives; rq is the state's
+// density, ri the inverse of the primitive one.  FP64 divisions bound the pass that
+// runs it: constants are divided once on the host.  art points at the cell (fields `cells` apart); one species has no
+// diffusion coefficient of its own (D* is never written and zero).
+template <typename F>
+__device__ __forceinline__ void rate_point(const RateConst& R, const double rq, const double ri, const double c,
+                                           const double cp, const double (&uv)[3], const F* __restrict__ art,
+                                           int64_t cells, int Ns, double& rate, double& rmin) {
+    rmin = jl_min(rmin, rq);
+    double acc = 0.0, dsum = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        if (!R.act[d]) continue;
+        acc += (fabs(uv[d]) + c) * R.idx[d];
+        dsum += R.idx[d] * R.idx[d];
+    }
+    const double D0 = R.mu0_Sc * ri;
+    double Dmax = D0;
+    if (Ns > 1)
+        for (int sp = 0; sp < Ns; ++sp) Dmax = jl_max(Dmax, D0 + double(art[cells * (A_D0 + sp)]));
+    const double nu = (R.mu0 + double(art[cells * A_MU]) + double(art[cells * A_BETA])) * ri +
+                      (R.mu0_Pr * cp + double(art[cells * A_KAPPA])) * ri / cp + Dmax;
+    acc += 2 * nu * dsum;
+    rate = jl_max(rate, acc);
 }
 
-#define GRID_STRIDE(idx, n) for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < (n); idx += (int64_t)gridDim.x * blockDim.x)
+// Block max / min of (rate, rmin) into part[2 b], part[2 b + 1] (max / min are
+// exact, so the order does not matter).
+__device__ __forceinline__ void rate_block_reduce(double rate, double rmin, double* __restrict__ part, int b) {
+    __shared__ double sr[kThreads], sm[kThreads];
+    sr[threadIdx.x] = rate;
+    sm[threadIdx.x] = rmin;
+    __syncthreads();
+    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+        if ((int)threadIdx.x < s) {
+            sr[threadIdx.x] = jl_max(sr[threadIdx.x], sr[threadIdx.x + s]);
+            sm[threadIdx.x] = jl_min(sm[threadIdx.x], sm[threadIdx.x + s]);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        part[2 * b] = sr[0];
+        part[2 * b + 1] = sm[0];
+    }
+}
 
 // _primitives!(::IdealMixture) (src/physics.jl:604-653) at the interior, and
 // _primitives!(::Nasa9Mixture) (src/physics.jl:501-570) when N9 (a separate
 // instantiation, so the ideal-gas kernel keeps its small register footprint).
 // PM (batched solves): the species constants are per batch member, mc[24 m ..]
 // = R_k, cv_k, cp_k (8 each) of member m = tmap[cell / 64].
-template <typename F, bool N9, bool PM = false>
-__global__ void k_primitives(const double* __restrict__ Q, F* __restrict__ prim, int64_t cells, int Ns, PhysConst pc,
-                             int esens, const double* __restrict__ mc = nullptr, const int* __restrict__ tmap = nullptr) {
+// RATE: the max_rate reduction of the cells just formed, per-block partials into
+// part.  As a pass of its own it read seven of these fields again: 443 us of a
+// 256^3 FP64 step, 200 us of a 192^3 mixed one.
+template <typename F, bool N9, bool PM = false, bool RATE = false>
+__global__ void __launch_bounds__(kThreads, RATE ? 3 : 4) k_primitives(const double* __restrict__ Q, F* __restrict__ prim, int64_t cells, int Ns, PhysConst pc,
+                             int esens, const double* __restrict__ mc = nullptr, const int* __restrict__ tmap = nullptr,
+                             const F* __restrict__ art = nullptr, double* __restrict__ part = nullptr,
+                             const RateConst rc = RateConst{}) {
+    double rate = 0.0, rmin = __longlong_as_double(0x7ff0000000000000LL);
     GRID_STRIDE(I, cells) {
         const double* mcI = nullptr;
         if constexpr (PM) mcI = mc + 24 * tmap[I >> 6];
         double rho = 0.0;
         for (int sp = 0; sp < Ns; ++sp) rho += Q[I + cells * sp];
+        const double rq = rho;
         F* out = prim + I;
-        if (N9 && rho > 0) {
-            const double ri = 1 / rho;
-            double Y[CLES_MAX_SPECIES];
-            double Rm = 0.0;
-            for (int sp = 0; sp < Ns; ++sp) {
-                Y[sp] = Q[I + cells * sp] * ri;
-                out[cells * (P_Y0 + sp)] = F(Y[sp]);
-                Rm += Y[sp] * pc.Rk[sp];
-            }
-            const double u = Q[I + cells * (Ns + 0)] * ri;
-            const double v = Q[I + cells * (Ns + 1)] * ri;
-            const double w = Q[I + cells * (Ns + 2)] * ri;
-            const double e = Q[I + cells * (Ns + 3)] * ri - 0.5 * (u * u + v * v + w * w);
-            const double T = n9_temperature(pc, Ns, e, Y);
-            double cpm = 0.0;
-            for (int sp = 0; sp < Ns; ++sp) cpm += Y[sp] * n9_cp(pc, sp, T);
-            const double cvm = cpm - Rm;
-            out[cells * P_RHO] = F(rho);
-            out[cells * P_U] = F(u);
-            out[cells * P_V] = F(v);
-            out[cells * P_W] = F(w);
-            out[cells * P_P] = F(rho * Rm * T);
-            out[cells * P_T] = F(T);
-            out[cells * P_C] = F(sqrt(jl_max((cpm / cvm) * Rm * T, 0.0)));
-            out[cells * P_CP] = F(cpm);
-            if (esens) {
-                const double r = jl_max(rho, 1e-300);
-                const double q1 = Q[I + cells * (Ns + 0)], q2 = Q[I + cells * (Ns + 1)], q3 = Q[I + cells * (Ns + 2)];
-                const double ke = 0.5 * (q1 * q1 + q2 * q2 + q3 * q3) / r;
-                out[cells * (P_Y0 + Ns)] = F((Q[I + cells * (Ns + 3)] - ke) / r);
-            }
-        } else if (rho > 0) {
-            const double ri = 1 / rho;
+        double u = 0, v = 0, w = 0, p = 1, T = 1, c = 1, cp = 1;   // placeholders of a cell without density
+        double er = 1.0, ri = 1.0;   // density of the energy sensor, inverse density
+        const double q1 = Q[I + cells * (Ns + 0)], q2 = Q[I + cells * (Ns + 1)], q3 = Q[I + cells * (Ns + 2)];
+        const double qe = Q[I + cells * (Ns + 3)];
+        if (rho > 0) {
+            ri = 1 / rho;
             double Rm = 0.0, cvm = 0.0;
+            double Y[N9 ? CLES_MAX_SPECIES : 1];
             for (int sp = 0; sp < Ns; ++sp) {
                 const double q = Q[I + cells * sp];
-                if constexpr (PM) {
+                if constexpr (N9) {
+                    Y[sp] = q * ri;
+                    Rm += Y[sp] * pc.Rk[sp];
+                } else if constexpr (PM) {
                     Rm += q * mcI[sp];
                     cvm += q * mcI[8 + sp];
                 } else {
@@ -160,57 +190,64 @@ __global__ void k_primitives(const double* __restrict__ Q, F* __restrict__ prim,
                 }
                 out[cells * (P_Y0 + sp)] = F(q * ri);
             }
-            Rm *= ri;
-            cvm *= ri;
-            const double u = Q[I + cells * (Ns + 0)] * ri;
-            const double v = Q[I + cells * (Ns + 1)] * ri;
-            const double w = Q[I + cells * (Ns + 2)] * ri;
-            const double e = Q[I + cells * (Ns + 3)] * ri - 0.5 * (u * u + v * v + w * w);
-            const double T = jl_max(e / cvm, 1e-300);
-            const double p = rho * Rm * T;
-            const double gm = 1 + Rm / cvm;
-            out[cells * P_RHO] = F(rho);
-            out[cells * P_U] = F(u);
-            out[cells * P_V] = F(v);
-            out[cells * P_W] = F(w);
-            out[cells * P_P] = F(p);
-            out[cells * P_T] = F(T);
-            out[cells * P_C] = F(sqrt(gm * Rm * T));
-            out[cells * P_CP] = F(cvm + Rm);
-            if (esens) {
-                // internal energy for the kappa* sensor (src/artificial.jl:322-330): rho floored, |m|^2/2rho
-                const double r = jl_max(rho, 1e-300);
-                const double q1 = Q[I + cells * (Ns + 0)], q2 = Q[I + cells * (Ns + 1)], q3 = Q[I + cells * (Ns + 2)];
-                const double ke = 0.5 * (q1 * q1 + q2 * q2 + q3 * q3) / r;
-                out[cells * (P_Y0 + Ns)] = F((Q[I + cells * (Ns + 3)] - ke) / r);
+            u = q1 * ri;
+            v = q2 * ri;
+            w = q3 * ri;
+            const double e = qe * ri - 0.5 * (u * u + v * v + w * w);
+            if constexpr (N9) {
+                T = n9_temperature(pc, Ns, e, Y);
+                cp = 0.0;
+                for (int sp = 0; sp < Ns; ++sp) cp += Y[sp] * n9_cp(pc, sp, T);
+                p = rho * Rm * T;
+                c = sqrt(jl_max((cp / (cp - Rm)) * Rm * T, 0.0));
+            } else {
+                Rm *= ri;
+                cvm *= ri;
+                T = jl_max(e / cvm, 1e-300);
+                p = rho * Rm * T;
+                const double gm = 1 + Rm / cvm;
+                c = sqrt(gm * Rm * T);
+                cp = cvm + Rm;
             }
+            er = jl_max(rho, 1e-300);
         } else {
-            out[cells * P_RHO] = F(1);
-            out[cells * P_U] = F(0);
-            out[cells * P_V] = F(0);
-            out[cells * P_W] = F(0);
-            out[cells * P_P] = F(1);
-            out[cells * P_T] = F(1);
-            out[cells * P_C] = F(1);
-            out[cells * P_CP] = F(1);
+            rho = 1;
             for (int sp = 0; sp < Ns; ++sp) out[cells * (P_Y0 + sp)] = F(sp == 0 ? 1.0 : 0.0);
-            if (esens) {
-                // placeholder density 1: the floor is max(1, 1e-300) = 1
-                const double q1 = Q[I + cells * (Ns + 0)], q2 = Q[I + cells * (Ns + 1)], q3 = Q[I + cells * (Ns + 2)];
-                const double ke = 0.5 * (q1 * q1 + q2 * q2 + q3 * q3) / 1.0;
-                out[cells * (P_Y0 + Ns)] = F((Q[I + cells * (Ns + 3)] - ke) / 1.0);
-            }
+        }
+        out[cells * P_RHO] = F(rho);
+        out[cells * P_U] = F(u);
+        out[cells * P_V] = F(v);
+        out[cells * P_W] = F(w);
+        out[cells * P_P] = F(p);
+        out[cells * P_T] = F(T);
+        out[cells * P_C] = F(c);
+        out[cells * P_CP] = F(cp);
+        if (esens) {
+            // internal energy for the kappa* sensor (src/artificial.jl:322-330): rho floored, |m|^2/2rho
+            const double ke = 0.5 * (q1 * q1 + q2 * q2 + q3 * q3) / er;
+            out[cells * (P_Y0 + Ns)] = F((qe - ke) / er);
+        }
+        if constexpr (RATE) {
+            // on the stored values, as a reduction over the fields would see them
+            const double uv[3] = {double(F(u)), double(F(v)), double(F(w))};
+            rate_point(rc, rq, sizeof(F) == 8 ? ri : 1 / double(F(rho)), double(F(c)), double(F(cp)), uv, art + I, cells, Ns,
+                       rate, rmin);
         }
     }
+    if constexpr (RATE) rate_block_reduce(rate, rmin, part, blockIdx.x);
 }
 
 // |S| = sqrt(S_ij S_ij) (src/artificial.jl:287-300); g[3d+j] = d u_j / d x_d.
-template <typename F>
+// DIMS: bit d set where the derivatives along d are not all zero (the others are
+// neither read here nor in k_fluxes: a 2-D grid saves a third of the gradients).
+// A template: tested at run time the loads are no longer issued together (k_fluxes
+// on 256^3 FP64 cells 766 -> 1572 us).
+template <typename F, int DIMS>
 __global__ void k_strain(const F* __restrict__ g, F* __restrict__ out, int64_t cells) {
     GRID_STRIDE(I, cells) {
         double gv[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) gv[k] = double(g[I + cells * k]);
+        for (int k = 0; k < 9; ++k) gv[k] = (DIMS >> (k / 3)) & 1 ? double(g[I + cells * k]) : 0.0;
         double ss = 0.0;
 #pragma unroll
         for (int b = 0; b < 3; ++b)
@@ -224,47 +261,16 @@ __global__ void k_strain(const F* __restrict__ g, F* __restrict__ out, int64_t c
 }
 
 // delta4_sum! (src/artificial.jl:67-94): sum_d h_d^p |(1,-4,6,-4,1) f| along d,
-// periodic wrap or clamping at closed edges.
-template <typename F>
-__global__ void k_delta4(const F* __restrict__ f, F* __restrict__ out, Grid3 g, double w0, double w1, double w2) {
-    const int64_t cells = (int64_t)g.n[0] * g.n[1] * g.n[2];
-    const double wd[3] = {w0, w1, w2};
-    const double D4[5] = {1.0, -4.0, 6.0, -4.0, 1.0};
-    const int64_t st[3] = {1, (int64_t)g.n[0], (int64_t)g.n[0] * g.n[1]};
-    GRID_STRIDE(I, cells) {
-        const int i = (int)(I % g.n[0]);
-        const int j = (int)((I / g.n[0]) % g.n[1]);
-        const int k = (int)(I / ((int64_t)g.n[0] * g.n[1]));
-        const int ijk[3] = {i, j, k};
-        double o = 0.0;
-        for (int d = 0; d < 3; ++d) {
-            if (!g.active[d]) continue;
-            const int nd = g.n[d];
-            const int il = ijk[d];
-            double acc = 0.0;
-#pragma unroll
-            for (int m = -2; m <= 2; ++m) {
-                int ilm = il + m;
-                if (g.periodic[d]) ilm = ilm < 0 ? ilm + nd : (ilm >= nd ? ilm - nd : ilm);
-                else ilm = ilm < 0 ? 0 : (ilm >= nd ? nd - 1 : ilm);
-                acc += D4[m + 2] * double(f[I + (int64_t)(ilm - il) * st[d]]);
-            }
-            o += wd[d] * fabs(acc);
-        }
-        out[I] = F(o);
-    }
-}
-
-// delta4_sum! for NF fields at once, tiled: a block of 256 threads covers
-// 32 x 16 (x, y) columns and walks z; each thread owns two neighbouring rows
-// of one x column.  The halo'd xy planes z0-2 .. z0+kZC+1 stream through a
-// ring of kRing planes in shared memory by cp.async (one commit group per
+// periodic wrap or clamping at closed edges, of several fields in one launch,
+// tiled: a block of 256 threads covers 32 x 16 (x, y) columns of one field and
+// walks nzc planes; each thread owns two neighbouring rows of one x column.  The
+// halo'd xy planes z0-2 .. z0+nzc+1 stream through a ring of kRing planes in shared memory by cp.async (one commit group per
 // plane); at plane z the x and y differences read plane z (the six column
 // values of a thread serve both rows' y differences) and the z difference a
 // register window of the thread's two columns, fed from plane z+2.  Eight
-// shared-memory reads a point and field.  Accumulation order per point is
+// shared-memory reads a point.  Accumulation order per point is
 // the reference's: out = 0; for d in x, y, z: out += w_d |sum_m D4_m f|.
-constexpr int kTX = kD4X, kTY = kD4Y, kZC = kD4Z;
+constexpr int kTX = kD4X, kTY = kD4Y;
 __device__ __forceinline__ int edge_index(int i, int n, int periodic) {
     if (periodic) return i < 0 ? i + n : (i >= n ? i - n : i);
     return i < 0 ? 0 : (i >= n ? n - 1 : i);
@@ -274,10 +280,6 @@ constexpr int kD4Threads = 256;
 constexpr int kPlane = (kTY + 4) * (kTX + 4);
 constexpr int kStage = (kPlane + kD4Threads - 1) / kD4Threads;   // staging slots a thread
 static_assert(kTX * kTY == 2 * kD4Threads, "two rows a thread");
-template <typename F, int NF>
-constexpr size_t delta4_smem() {
-    return sizeof(F) * (size_t)kRing * NF * kPlane;
-}
 __device__ __forceinline__ unsigned d4_smem_addr(const void* p) {
     return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
@@ -290,15 +292,12 @@ __device__ __forceinline__ void d4_cp_async(F* dst, const F* src) {
 }
 __device__ __forceinline__ void d4_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-template <typename F, int NF>
-__device__ __forceinline__ void delta4_tile(const F* __restrict__ f0, const F* __restrict__ f1, F* __restrict__ o0,
-                                            F* __restrict__ o1, const Grid3& g, const Weights3& w0,
-                                            const Weights3& w1, const int x0, const int y0, const int z0,
-                                            F* __restrict__ ring) {
+template <typename F>
+__device__ __forceinline__ void delta4_tile(const F* __restrict__ f0, F* __restrict__ o0, const Grid3& g,
+                                            const Weights3& w0, const int x0, const int y0, const int z0,
+                                            const int nzc) {
+    __shared__ __align__(16) F ring[kRing * kPlane];
     constexpr int TW = kTX + 4;
-    const F* fs[2] = {f0, f1};
-    F* os[2] = {o0, o1};
-    const Weights3 ws[2] = {w0, w1};
     const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
     const int64_t sy = nx, sz = (int64_t)nx * ny;
     const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;
@@ -319,21 +318,18 @@ __device__ __forceinline__ void delta4_tile(const F* __restrict__ f0, const F* _
         const int gy = g.active[1] ? edge_index(y0 - 2 + hy, ny, g.periodic[1]) : min(y0 - 2 + hy < 0 ? 0 : y0 - 2 + hy, ny - 1);
         soff_g[s] = (int64_t)gx + (int64_t)gy * sy;
     }
-    const int zend = min(z0 + kZC, nz);
+    const int zend = min(z0 + nzc, nz);
     // plane r of the block (r = 0 is z0 - 2) into ring slot r % kRing; planes
     // past the last one any output reads are left out (empty group)
     const int rlast = zact ? (zend - 1 + 2) - (z0 - 2) : 2;
-    auto slot = [&](int r) { return ring + (size_t)(r % kRing) * NF * kPlane; };
+    auto slot = [&](int r) { return ring + (r % kRing) * kPlane; };
     auto issue = [&](int r) {
         if (r <= rlast) {
             const int zz = zact ? edge_index(z0 - 2 + r, nz, g.periodic[2]) : 0;
             F* sl = slot(r);
 #pragma unroll
-            for (int f = 0; f < NF; ++f)
-#pragma unroll
-                for (int s = 0; s < kStage; ++s)
-                    if (sv[s])
-                        d4_cp_async(sl + f * kPlane + threadIdx.x + kD4Threads * s, fs[f] + soff_g[s] + (int64_t)zz * sz);
+            for (int s = 0; s < kStage; ++s)
+                if (sv[s]) d4_cp_async(sl + threadIdx.x + kD4Threads * s, f0 + soff_g[s] + (int64_t)zz * sz);
         }
         d4_commit();
     };
@@ -342,16 +338,14 @@ __device__ __forceinline__ void delta4_tile(const F* __restrict__ f0, const F* _
     // planes 0 .. 5; the z window starts with planes 0 .. 3 (z0-2 .. z0+1)
 #pragma unroll
     for (int r = 0; r < kRing; ++r) issue(r);
-    F zw[NF][2][5];
+    F zw[2][5];
     asm volatile("cp.async.wait_group 2;" ::: "memory");
     __syncthreads();
     if (zact) {
 #pragma unroll
-        for (int f = 0; f < NF; ++f)
+        for (int q = 0; q < 4; ++q)
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int t = 0; t < 2; ++t) zw[f][t][q + 1] = slot(q)[f * kPlane + cofs + t * TW];
+            for (int t = 0; t < 2; ++t) zw[t][q + 1] = slot(q)[cofs + t * TW];
     }
     for (int z = z0; z < zend; ++z) {
         const int rz = z - z0 + 2;
@@ -363,15 +357,14 @@ __device__ __forceinline__ void delta4_tile(const F* __restrict__ f0, const F* _
         issue(rz + 4);
         const F* pl = slot(rz);
         const F* pc = slot(rz + 2);
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            const F* t0 = pl + f * kPlane;
+        {
+            const F* t0 = pl;
             if (zact) {
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) zw[f][t][q] = zw[f][t][q + 1];
-                    zw[f][t][4] = pc[f * kPlane + cofs + t * TW];
+                    for (int q = 0; q < 4; ++q) zw[t][q] = zw[t][q + 1];
+                    zw[t][4] = pc[cofs + t * TW];
                 }
             }
             // the column x: tile rows 2ty .. 2ty+5 (both rows' y stencils)
@@ -387,34 +380,33 @@ __device__ __forceinline__ void delta4_tile(const F* __restrict__ f0, const F* _
                     double acc = 0.0;
 #pragma unroll
                     for (int m = 0; m < 5; ++m) acc += D4[m] * double(m == 2 ? cy[2 + t] : row[m]);
-                    o += ws[f].w[0] * fabs(acc);
+                    o += w0.w[0] * fabs(acc);
                 }
                 if (g.active[1]) {
                     double acc = 0.0;
 #pragma unroll
                     for (int m = 0; m < 5; ++m) acc += D4[m] * double(cy[t + m]);
-                    o += ws[f].w[1] * fabs(acc);
+                    o += w0.w[1] * fabs(acc);
                 }
                 if (zact) {
                     double acc = 0.0;
 #pragma unroll
-                    for (int m = 0; m < 5; ++m) acc += D4[m] * double(zw[f][t][m]);
-                    o += ws[f].w[2] * fabs(acc);
+                    for (int m = 0; m < 5; ++m) acc += D4[m] * double(zw[t][m]);
+                    o += w0.w[2] * fabs(acc);
                 }
-                os[f][x + (int64_t)(ya + t) * sy + (int64_t)z * sz] = F(o);
+                o0[x + (int64_t)(ya + t) * sy + (int64_t)z * sz] = F(o);
             }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-template <typename F, int NF>
-__global__ void __launch_bounds__(kD4Threads) k_delta4_tiled(const F* __restrict__ f0, const F* __restrict__ f1,
-                                                           F* __restrict__ o0, F* __restrict__ o1, Grid3 g,
-                                                           Weights3 w0, Weights3 w1) {
-    extern __shared__ __align__(16) unsigned char d4_raw[];
-    delta4_tile<F, NF>(f0, f1, o0, o1, g, w0, w1, blockIdx.x * kTX, blockIdx.y * kTY, blockIdx.z * kZC,
-                       reinterpret_cast<F*>(d4_raw));
+template <typename F>
+__global__ void __launch_bounds__(kD4Threads) k_delta4(const D4Set<F> fs, Grid3 g, Weights3 h, int nzc, int nchunks) {
+    const int f = blockIdx.z / nchunks, zc = blockIdx.z - f * nchunks;
+    Weights3 w;
+    for (int d = 0; d < 3; ++d) w.w[d] = fs.p[f] == 2 ? h.w[d] * h.w[d] : h.w[d];
+    delta4_tile<F>(fs.in[f], fs.out[f], g, w, blockIdx.x * kTX, blockIdx.y * kTY, zc * nzc, nzc);
 }
 
 // delta4_sum! of one or two fields on a rank's block of a decomposed grid
@@ -479,33 +471,17 @@ __device__ __forceinline__ double compression_switch(const double* gv) {
     return div * div / (div * div + w1 * w1 + w2 * w2 + w3 * w3 + 1e-32);
 }
 
-// mu*, beta* from the smoothed strain sensor (src/artificial.jl:306-313),
-// optional gating (gate_beta!, :164-175).
+// mu*, beta* (optionally gated), kappa* and every D*_k from the smoothed sensors
+// (strain, internal energy, Y_1 ..; fields `cells` apart) in one pass
+// (src/artificial.jl:306-313, :334-341, :348-356).
 template <typename F>
-__global__ void k_mu_beta(const F* __restrict__ sensor, const F* __restrict__ prim, const F* __restrict__ g,
-                          F* __restrict__ art, int64_t cells, double C_mu, double C_beta, int gate) {
-    GRID_STRIDE(I, cells) {
-        const double rs = double(prim[I + cells * P_RHO]) * jl_max(double(sensor[I]), 0.0);
-        double beta = C_beta * rs;
-        if (gate) {
-            double gv[9];
-            for (int k = 0; k < 9; ++k) gv[k] = double(g[I + cells * k]);
-            beta *= compression_switch(gv);
-        }
-        art[I + cells * A_MU] = F(C_mu * rs);
-        art[I + cells * A_BETA] = F(beta);
-    }
-}
-
-// mu*, beta* (optionally gated) and kappa* from the two smoothed sensors in one
-// pass (src/artificial.jl:306-313 and :334-341).
-template <typename F>
-__global__ void k_art_coef(const F* __restrict__ s_strain, const F* __restrict__ s_energy, const F* __restrict__ prim,
-                           const F* __restrict__ g, F* __restrict__ art, int64_t cells, double C_mu, double C_beta,
-                           double C_kappa, int gate) {
+__global__ void k_art_coef(const F* __restrict__ sens, const F* __restrict__ prim, const F* __restrict__ g,
+                           F* __restrict__ art, int64_t cells, int Ns, double C_mu, double C_beta, double C_kappa,
+                           double C_D, int gate) {
     GRID_STRIDE(I, cells) {
         const double rho = double(prim[I + cells * P_RHO]);
-        const double rs = rho * jl_max(double(s_strain[I]), 0.0);
+        const double c = double(prim[I + cells * P_C]);
+        const double rs = rho * jl_max(double(sens[I]), 0.0);
         double beta = C_beta * rs;
         if (gate) {
             double gv[9];
@@ -514,8 +490,11 @@ __global__ void k_art_coef(const F* __restrict__ s_strain, const F* __restrict__
         }
         art[I + cells * A_MU] = F(C_mu * rs);
         art[I + cells * A_BETA] = F(beta);
-        const double scale = rho * double(prim[I + cells * P_C]) / jl_max(double(prim[I + cells * P_T]), 2.220446049250313e-16);
-        art[I + cells * A_KAPPA] = F(C_kappa * scale * jl_max(double(s_energy[I]), 0.0));
+        const double scale = rho * c / jl_max(double(prim[I + cells * P_T]), 2.220446049250313e-16);
+        art[I + cells * A_KAPPA] = F(C_kappa * scale * jl_max(double(sens[I + cells]), 0.0));
+        if (Ns > 1)
+            for (int sp = 0; sp < Ns; ++sp)
+                art[I + cells * (A_D0 + sp)] = F(C_D * c * jl_max(double(sens[I + cells * (2 + sp)]), 0.0));
     }
 }
 
@@ -539,44 +518,16 @@ __global__ void k_beta_dilatation(const F* __restrict__ sensor, const F* __restr
     }
 }
 
-// internal energy e = (E - |m|^2/2rho)/rho with rho floored (src/artificial.jl:322-330)
-template <typename F>
-__global__ void k_energy(const double* __restrict__ Q, const F* __restrict__ prim, F* __restrict__ out, int64_t cells,
-                         int Ns) {
-    GRID_STRIDE(I, cells) {
-        const double r = jl_max(double(prim[I + cells * P_RHO]), 1e-300);
-        const double q1 = Q[I + cells * (Ns + 0)], q2 = Q[I + cells * (Ns + 1)], q3 = Q[I + cells * (Ns + 2)];
-        const double ke = 0.5 * (q1 * q1 + q2 * q2 + q3 * q3) / r;
-        out[I] = F((Q[I + cells * (Ns + 3)] - ke) / r);
-    }
-}
-
-// kappa* = C_kappa (rho c / max(T, eps)) max(sensor, 0) (src/artificial.jl:334-341, src/physics.jl:155-156)
-template <typename F>
-__global__ void k_kappa(const F* __restrict__ sensor, const F* __restrict__ prim, F* __restrict__ art, int64_t cells,
-                        double C_kappa) {
-    GRID_STRIDE(I, cells) {
-        const double scale = double(prim[I + cells * P_RHO]) * double(prim[I + cells * P_C]) /
-                             jl_max(double(prim[I + cells * P_T]), 2.220446049250313e-16);
-        art[I + cells * A_KAPPA] = F(C_kappa * scale * jl_max(double(sensor[I]), 0.0));
-    }
-}
-
-// D*_k = C_D c max(sensor_k, 0) (src/artificial.jl:348-356)
-template <typename F>
-__global__ void k_dart(const F* __restrict__ sensor, const F* __restrict__ prim, F* __restrict__ art, int64_t cells,
-                       double C_D, int sp) {
-    GRID_STRIDE(I, cells) {
-        art[I + cells * (A_D0 + sp)] = F(C_D * double(prim[I + cells * P_C]) * jl_max(double(sensor[I]), 0.0));
-    }
-}
-
 // _assemble_fluxes! (src/rhs.jl:495-556).  gty[d*(1+Ns) + 0] = dT/dx_d,
 // gty[d*(1+Ns) + 1 + k] = dY_k/dx_d; flux[d*ncons + c].
 // SINGLE (one species): the species diffusion flux rho D dY (Y - 1) is zero in
 // exact arithmetic (Y = 1) and below ~1e-30 of the momentum flux in FP64, so it
 // is taken as 0 and dY/dx_d is neither computed nor read (gty holds dT only).
-template <typename F, bool SINGLE, bool N9, bool GEO, bool PM = false>
+// DIMS: the active dimensions; the flux of a collapsed one is neither formed nor
+// stored, and off curvilinear grids (GEO adds curvature terms to them) its
+// gradients are zero and not read.  Two species on 2048 x 1024 cells: 169 us with
+// all three directions.
+template <typename F, bool SINGLE, bool N9, bool GEO, bool PM = false, int DIMS = 7>
 __global__ void k_fluxes(const double* __restrict__ Q, const F* __restrict__ prim, const F* __restrict__ g,
                          const F* __restrict__ gty, const F* __restrict__ art, F* __restrict__ flux, int64_t cells,
                          int Ns, PhysConst pc, double mu0, double Pr, double Sc, Geom G,
@@ -598,7 +549,7 @@ __global__ void k_fluxes(const double* __restrict__ Q, const F* __restrict__ pri
 #define CLES_AF(v) (GEO ? __dmul_rn(ad, (v)) : (v))
         double gv[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) gv[k] = double(g[I + cells * k]);
+        for (int k = 0; k < 9; ++k) gv[k] = GEO || ((DIMS >> (k / 3)) & 1) ? double(g[I + cells * k]) : 0.0;
         const double r = double(prim[I + cells * P_RHO]);
         const double uv[3] = {double(prim[I + cells * P_U]), double(prim[I + cells * P_V]), double(prim[I + cells * P_W])};
         const double p = double(prim[I + cells * P_P]);
@@ -618,6 +569,7 @@ __global__ void k_fluxes(const double* __restrict__ Q, const F* __restrict__ pri
         const double tau[3][3] = {{t11, t12, t13}, {t12, t22, t23}, {t13, t23, t33}};
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
+            if (!((DIMS >> d) & 1)) continue;   // no divergence along a collapsed dimension
             const double ud = uv[d];
             const double ad = area[d];
             const double* td = tau[d];
@@ -689,69 +641,6 @@ __global__ void k_lsrk(double* __restrict__ Q, double* __restrict__ du, const F*
         du[I] = v;
         Q[I] += B * v;
     }
-}
-
-// The max_rate contribution of cell I (src/timestep.jl:125-175), Cartesian;
-// fields are `cells` elements apart.
-template <typename F>
-__device__ __forceinline__ void rate_cell(const double* __restrict__ Q, const F* __restrict__ prim,
-                                          const F* __restrict__ art, int64_t I, int64_t cells, int Ns,
-                                          const double idx[3], const int act[3], double mu0, double Pr, double Sc,
-                                          double& rate, double& rmin) {
-    {
-        double rq = 0.0;
-        for (int sp = 0; sp < Ns; ++sp) rq += Q[I + cells * sp];
-        rmin = jl_min(rmin, rq);
-        const double r = double(prim[I + cells * P_RHO]);
-        const double ri = 1 / r;
-        const double c = double(prim[I + cells * P_C]);
-        const double cp = double(prim[I + cells * P_CP]);
-        const double uv[3] = {double(prim[I + cells * P_U]), double(prim[I + cells * P_V]), double(prim[I + cells * P_W])};
-        double acc = 0.0, dsum = 0.0;
-        for (int d = 0; d < 3; ++d) {
-            if (!act[d]) continue;
-            acc += (fabs(uv[d]) + c) * idx[d];
-            dsum += idx[d] * idx[d];
-        }
-        double Dmax = mu0 / (Sc * r);
-        for (int sp = 0; sp < Ns; ++sp) Dmax = jl_max(Dmax, mu0 / (Sc * r) + double(art[I + cells * (A_D0 + sp)]));
-        const double nu = (mu0 + double(art[I + cells * A_MU]) + double(art[I + cells * A_BETA])) * ri +
-                          (mu0 * cp / Pr + double(art[I + cells * A_KAPPA])) * ri / cp + Dmax;
-        acc += 2 * nu * dsum;
-        rate = jl_max(rate, acc);
-    }
-}
-
-// Block max / min of (rate, rmin) into part[2 b], part[2 b + 1] (max / min are
-// exact, so the order does not matter).
-__device__ __forceinline__ void rate_block_reduce(double rate, double rmin, double* __restrict__ part, int b) {
-    __shared__ double sr[kThreads], sm[kThreads];
-    sr[threadIdx.x] = rate;
-    sm[threadIdx.x] = rmin;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) {
-            sr[threadIdx.x] = jl_max(sr[threadIdx.x], sr[threadIdx.x + s]);
-            sm[threadIdx.x] = jl_min(sm[threadIdx.x], sm[threadIdx.x + s]);
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        part[2 * b] = sr[0];
-        part[2 * b + 1] = sm[0];
-    }
-}
-
-// max_rate per-block partials (src/timestep.jl:125-175), Cartesian.
-template <typename F>
-__global__ void k_rate_partial(const double* __restrict__ Q, const F* __restrict__ prim, const F* __restrict__ art,
-                               double* __restrict__ part, int64_t cells, int Ns, double idx0, double idx1, double idx2,
-                               int a0, int a1, int a2, double mu0, double Pr, double Sc) {
-    double rate = 0.0, rmin = __longlong_as_double(0x7ff0000000000000LL);
-    const double idx[3] = {idx0, idx1, idx2};
-    const int act[3] = {a0, a1, a2};
-    GRID_STRIDE(I, cells) rate_cell(Q, prim, art, I, cells, Ns, idx, act, mu0, Pr, Sc, rate, rmin);
-    rate_block_reduce(rate, rmin, part, blockIdx.x);
 }
 
 __global__ void k_rate_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
@@ -1034,11 +923,6 @@ __global__ void k_gather_interior(const double* __restrict__ padded, double* __r
 }
 
 template <typename F>
-__global__ void k_convert(const double* __restrict__ a, F* __restrict__ b, int64_t n) {
-    GRID_STRIDE(I, n) b[I] = F(a[I]);
-}
-
-template <typename F>
 __global__ void k_to_double(const F* __restrict__ a, double* __restrict__ b, int64_t n) {
     GRID_STRIDE(I, n) b[I] = double(a[I]);
 }
@@ -1081,21 +965,15 @@ __global__ void k_clock_after(double* __restrict__ clk, ClockConst c) {
 }
 
 // ---- batched forms over the grids of a batch --------------------------------
-template <typename F, int NF>
-__global__ void __launch_bounds__(kD4Threads) k_delta4_batch(const F* __restrict__ f0, const F* __restrict__ f1,
-                                                           F* __restrict__ o0, F* __restrict__ o1, int p0, int p1,
-                                                           const BatchGrid* __restrict__ grids,
+template <typename F>
+__global__ void __launch_bounds__(kD4Threads) k_delta4_batch(const D4Set<F> fs, const BatchGrid* __restrict__ grids,
                                                            const BatchTile* __restrict__ tiles) {
-    extern __shared__ __align__(16) unsigned char d4_raw[];
     const BatchTile t = tiles[blockIdx.x];
     const BatchGrid& G = grids[t.grid];
-    Weights3 w0, w1;
-    for (int d = 0; d < 3; ++d) {
-        w0.w[d] = p0 == 2 ? G.h[d] * G.h[d] : G.h[d];
-        w1.w[d] = p1 == 2 ? G.h[d] * G.h[d] : G.h[d];
-    }
-    delta4_tile<F, NF>(f0 + G.off, f1 ? f1 + G.off : nullptr, o0 + G.off, o1 ? o1 + G.off : nullptr, G.g, w0, w1,
-                       t.x0, t.y0, t.z0, reinterpret_cast<F*>(d4_raw));
+    const int f = blockIdx.y;
+    Weights3 w;
+    for (int d = 0; d < 3; ++d) w.w[d] = fs.p[f] == 2 ? G.h[d] * G.h[d] : G.h[d];
+    delta4_tile<F>(fs.in[f] + G.off, fs.out[f] + G.off, G.g, w, t.x0, t.y0, t.z0, kD4Z);
 }
 
 template <typename F>
@@ -1105,13 +983,21 @@ __global__ void k_rate_batch_partial(const double* __restrict__ Q, const F* __re
                                      int Ns, double mu0, double Pr, double Sc) {
     const BatchChunk ch = chunks[blockIdx.x];
     const BatchGrid& G = grids[ch.grid];
-    double idx[3];
-    int act[3];
-    for (int d = 0; d < 3; ++d) { idx[d] = 1.0 / G.h[d]; act[d] = G.g.active[d]; }
+    RateConst R;
+    for (int d = 0; d < 3; ++d) { R.idx[d] = 1.0 / G.h[d]; R.act[d] = G.g.active[d]; }
+    R.mu0 = mu0;
+    R.mu0_Pr = mu0 / Pr;
+    R.mu0_Sc = mu0 / Sc;
     double rate = 0.0, rmin = __longlong_as_double(0x7ff0000000000000LL);
     const int64_t end = min(ch.c0 + (int64_t)kBatchChunk, G.cells);
-    for (int64_t c = ch.c0 + threadIdx.x; c < end; c += blockDim.x)
-        rate_cell(Q, prim, art, G.off + c, ct, Ns, idx, act, mu0, Pr, Sc, rate, rmin);
+    for (int64_t c = ch.c0 + threadIdx.x; c < end; c += blockDim.x) {
+        const int64_t I = G.off + c;
+        double rq = 0.0;
+        for (int sp = 0; sp < Ns; ++sp) rq += Q[I + ct * sp];
+        const double uv[3] = {double(prim[I + ct * P_U]), double(prim[I + ct * P_V]), double(prim[I + ct * P_W])};
+        rate_point(R, rq, 1 / double(prim[I + ct * P_RHO]), double(prim[I + ct * P_C]), double(prim[I + ct * P_CP]), uv,
+                   art + I, ct, Ns, rate, rmin);
+    }
     rate_block_reduce(rate, rmin, part, blockIdx.x);
 }
 
@@ -1170,18 +1056,10 @@ void clock_before(double* clk, const double* rate_rmin, const ClockConst& c, cud
     check_launch("k_clock_before");
 }
 template <typename F>
-void BatchOps<F>::delta4(const F* f0, const F* f1, F* o0, F* o1, int p0, int p1, const BatchGrid* grids,
-                         const BatchTile* tiles, int ntiles, int64_t, cudaStream_t st) {
-    if (ntiles <= 0) return;
-    if (f1) {
-        constexpr size_t sm = delta4_smem<F, 2>();
-        set_smem_attr(k_delta4_batch<F, 2>, sm);
-        k_delta4_batch<F, 2><<<ntiles, kD4Threads, sm, st>>>(f0, f1, o0, o1, p0, p1, grids, tiles);
-    } else {
-        constexpr size_t sm = delta4_smem<F, 1>();
-        set_smem_attr(k_delta4_batch<F, 1>, sm);
-        k_delta4_batch<F, 1><<<ntiles, kD4Threads, sm, st>>>(f0, f1, o0, o1, p0, p1, grids, tiles);
-    }
+void BatchOps<F>::delta4(const D4Set<F>& fs, const BatchGrid* grids, const BatchTile* tiles, int ntiles,
+                         cudaStream_t st) {
+    if (ntiles <= 0 || fs.n <= 0) return;
+    k_delta4_batch<F><<<dim3((unsigned)ntiles, (unsigned)fs.n), kD4Threads, 0, st>>>(fs, grids, tiles);
     count_launch();
     check_launch("k_delta4_batch");
 }
@@ -1199,19 +1077,28 @@ void BatchOps<F>::rate_clock(const double* Q, const F* prim, const F* art, const
 template <typename F>
 void BatchOps<F>::primitives(const double* Q, F* prim, int64_t ct, int Ns, const PhysConst& pc, int esens,
                              const double* mc, const int* tmap, cudaStream_t st) {
-    LAUNCH((k_primitives<F, false, true>), ct, st, Q, prim, ct, Ns, pc, esens, mc, tmap);
+    LAUNCH((k_primitives<F, false, true>), ct, st, Q, prim, ct, Ns, pc, esens, mc, tmap, nullptr, nullptr, RateConst{});
 }
+// k_fluxes for the active dimensions: 1-D and 2-D grids along x and y have their
+// own instantiations, any other set runs all three directions (the gradients of a
+// collapsed dimension are zero, its flux is not read)
+#define LAUNCH_FLUXES(F, SINGLE, N9, GEO, PM, n, st, ...)                                \
+    do {                                                                                 \
+        if (dims == 1) LAUNCH((k_fluxes<F, SINGLE, N9, GEO, PM, 1>), n, st, __VA_ARGS__); \
+        else if (dims == 3) LAUNCH((k_fluxes<F, SINGLE, N9, GEO, PM, 3>), n, st, __VA_ARGS__); \
+        else LAUNCH((k_fluxes<F, SINGLE, N9, GEO, PM, 7>), n, st, __VA_ARGS__);           \
+    } while (0)
 template <typename F>
 void BatchOps<F>::fluxes(const double* Q, const F* prim, const F* g, const F* gty, const F* art, F* flux, int64_t ct,
-                         int Ns, const PhysConst& pc, double mu0, double Pr, double Sc, const double* mc,
+                         int Ns, const PhysConst& pc, double mu0, double Pr, double Sc, int dims, const double* mc,
                          const int* tmap, cudaStream_t st) {
     const Geom G{};
     if (Ns == 1)
-        LAUNCH((k_fluxes<F, true, false, false>), ct, st, Q, prim, g, gty, art, flux, ct, Ns, pc, mu0, Pr, Sc, G,
-               nullptr, nullptr);
+        LAUNCH_FLUXES(F, true, false, false, false, ct, st, Q, prim, g, gty, art, flux, ct, Ns, pc, mu0, Pr, Sc, G,
+                      nullptr, nullptr);
     else
-        LAUNCH((k_fluxes<F, false, false, false, true>), ct, st, Q, prim, g, gty, art, flux, ct, Ns, pc, mu0, Pr, Sc,
-               G, mc, tmap);
+        LAUNCH_FLUXES(F, false, false, false, true, ct, st, Q, prim, g, gty, art, flux, ct, Ns, pc, mu0, Pr, Sc, G, mc,
+                      tmap);
 }
 template <typename F>
 void BatchOps<F>::lsrk(double* Q, double* du, const F* dQ, int64_t ct, int ncons, const int* tmap,
@@ -1245,27 +1132,23 @@ void clock_after(double* clk, const ClockConst& c, cudaStream_t st) {
 template <typename F>
 void Pointwise<F>::primitives(const double* Q, F* prim, int64_t cells, int Ns, const PhysConst& pc, cudaStream_t st,
                               int esens) {
-    if (pc.eos == CLES_EOS_NASA9) LAUNCH((k_primitives<F, true>), cells, st, Q, prim, cells, Ns, pc, esens, nullptr, nullptr);
-    else LAUNCH((k_primitives<F, false>), cells, st, Q, prim, cells, Ns, pc, esens, nullptr, nullptr);
+    if (pc.eos == CLES_EOS_NASA9) LAUNCH((k_primitives<F, true>), cells, st, Q, prim, cells, Ns, pc, esens, nullptr, nullptr, nullptr, nullptr, RateConst{});
+    else LAUNCH((k_primitives<F, false>), cells, st, Q, prim, cells, Ns, pc, esens, nullptr, nullptr, nullptr, nullptr, RateConst{});
 }
+// Planes a block walks: 32 (the four planes of run-in cost an eighth), fewer
+// where the launch would leave the SMs with less than four blocks of 256 threads
+// each; at least 8.  Two fields of 64^3: 16 blocks and 35 us a launch with 32.
 template <typename F>
-void Pointwise<F>::delta4_tiled(const F* f0, const F* f1, F* o0, F* o1, const Grid3& g, const double w0[3],
-                                const double w1[3], cudaStream_t st) {
-    dim3 grid((unsigned)((g.n[0] + kTX - 1) / kTX), (unsigned)((g.n[1] + kTY - 1) / kTY),
-              (unsigned)((g.n[2] + kZC - 1) / kZC));
-    Weights3 a{{w0[0], w0[1], w0[2]}}, b{{0.0, 0.0, 0.0}};
-    if (f1) {
-        b = Weights3{{w1[0], w1[1], w1[2]}};
-        constexpr size_t sm = delta4_smem<F, 2>();
-        set_smem_attr(k_delta4_tiled<F, 2>, sm);
-        k_delta4_tiled<F, 2><<<grid, kD4Threads, sm, st>>>(f0, f1, o0, o1, g, a, b);
-    } else {
-        constexpr size_t sm = delta4_smem<F, 1>();
-        set_smem_attr(k_delta4_tiled<F, 1>, sm);
-        k_delta4_tiled<F, 1><<<grid, kD4Threads, sm, st>>>(f0, nullptr, o0, nullptr, g, a, b);
-    }
+void Pointwise<F>::delta4(const D4Set<F>& fs, const Grid3& g, const double h[3], cudaStream_t st) {
+    if (fs.n <= 0) return;
+    const int bx = (g.n[0] + kTX - 1) / kTX, by = (g.n[1] + kTY - 1) / kTY;
+    int nzc = 32;
+    while (nzc > 8 && (int64_t)bx * by * ((g.n[2] + nzc - 1) / nzc) * fs.n < 4 * num_sms()) nzc /= 2;
+    const int nchunks = (g.n[2] + nzc - 1) / nzc;
+    const dim3 grid((unsigned)bx, (unsigned)by, (unsigned)(nchunks * fs.n));
+    k_delta4<F><<<grid, kD4Threads, 0, st>>>(fs, g, Weights3{{h[0], h[1], h[2]}}, nzc, nchunks);
     count_launch();
-    check_launch("k_delta4_tiled");
+    check_launch("k_delta4");
 }
 template <typename F>
 void Pointwise<F>::delta4_halo(const F* f0, const F* f1, F* o0, F* o1, const Grid3& g, const double w0[3],
@@ -1280,23 +1163,17 @@ void Pointwise<F>::delta4_halo(const F* f0, const F* f1, F* o0, F* o1, const Gri
     }
 }
 template <typename F>
-void Pointwise<F>::art_coef(const F* s_strain, const F* s_energy, const F* prim, const F* g, F* art, int64_t cells,
-                            double C_mu, double C_beta, double C_kappa, int gate, cudaStream_t st) {
-    LAUNCH(k_art_coef<F>, cells, st, s_strain, s_energy, prim, g, art, cells, C_mu, C_beta, C_kappa, gate);
+void Pointwise<F>::art_coef(const F* sens, const F* prim, const F* g, F* art, int64_t cells, int Ns, double C_mu,
+                            double C_beta, double C_kappa, double C_D, int gate, cudaStream_t st) {
+    LAUNCH(k_art_coef<F>, cells, st, sens, prim, g, art, cells, Ns, C_mu, C_beta, C_kappa, C_D, gate);
 }
 template <typename F>
-void Pointwise<F>::strain(const F* g, F* out, int64_t cells, cudaStream_t st) {
-    LAUNCH(k_strain<F>, cells, st, g, out, cells);
-}
-template <typename F>
-void Pointwise<F>::delta4(const F* f, F* out, const Grid3& g, const double wd[3], cudaStream_t st) {
-    const int64_t cells = (int64_t)g.n[0] * g.n[1] * g.n[2];
-    LAUNCH(k_delta4<F>, cells, st, f, out, g, wd[0], wd[1], wd[2]);
-}
-template <typename F>
-void Pointwise<F>::mu_beta(const F* sensor, const F* prim, const F* g, F* art, int64_t cells, double C_mu,
-                           double C_beta, int gate, cudaStream_t st) {
-    LAUNCH(k_mu_beta<F>, cells, st, sensor, prim, g, art, cells, C_mu, C_beta, gate);
+void Pointwise<F>::strain(const F* g, F* out, int64_t cells, int dims, cudaStream_t st) {
+    switch (dims) {
+        case 1: LAUNCH((k_strain<F, 1>), cells, st, g, out, cells); break;
+        case 3: LAUNCH((k_strain<F, 3>), cells, st, g, out, cells); break;
+        default: LAUNCH((k_strain<F, 7>), cells, st, g, out, cells);
+    }
 }
 template <typename F>
 void Pointwise<F>::dilatation(const F* g, F* div, F* sw, int64_t cells, cudaStream_t st) {
@@ -1308,39 +1185,33 @@ void Pointwise<F>::beta_dilatation(const F* sensor, const F* prim, const F* sw, 
     LAUNCH(k_beta_dilatation<F>, cells, st, sensor, prim, sw, art, cells, C_beta);
 }
 template <typename F>
-void Pointwise<F>::energy(const double* Q, const F* prim, F* out, int64_t cells, int Ns, cudaStream_t st) {
-    LAUNCH(k_energy<F>, cells, st, Q, prim, out, cells, Ns);
-}
-template <typename F>
-void Pointwise<F>::kappa(const F* sensor, const F* prim, F* art, int64_t cells, double C_kappa, cudaStream_t st) {
-    LAUNCH(k_kappa<F>, cells, st, sensor, prim, art, cells, C_kappa);
-}
-template <typename F>
-void Pointwise<F>::dart(const F* sensor, const F* prim, F* art, int64_t cells, double C_D, int sp, cudaStream_t st) {
-    LAUNCH(k_dart<F>, cells, st, sensor, prim, art, cells, C_D, sp);
-}
-template <typename F>
 void Pointwise<F>::fluxes(const double* Q, const F* prim, const F* g, const F* gty, const F* art, F* flux,
-                          int64_t cells, int Ns, const PhysConst& pc, double mu0, double Pr, double Sc,
+                          int64_t cells, int Ns, const PhysConst& pc, double mu0, double Pr, double Sc, int dims,
                           cudaStream_t st) {
     const Geom G{};
     if (Ns == 1)
-        LAUNCH((k_fluxes<F, true, false, false>), cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G, nullptr, nullptr);
+        LAUNCH_FLUXES(F, true, false, false, false, cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G,
+                      nullptr, nullptr);
     else if (pc.eos == CLES_EOS_NASA9)
-        LAUNCH((k_fluxes<F, false, true, false>), cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G, nullptr, nullptr);
+        LAUNCH_FLUXES(F, false, true, false, false, cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G,
+                      nullptr, nullptr);
     else
-        LAUNCH((k_fluxes<F, false, false, false>), cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G, nullptr, nullptr);
+        LAUNCH_FLUXES(F, false, false, false, false, cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc,
+                      G, nullptr, nullptr);
 }
 template <typename F>
 void Pointwise<F>::fluxes_geo(const double* Q, const F* prim, const F* g, const F* gty, const F* art, F* flux,
                               int64_t cells, int Ns, const PhysConst& pc, double mu0, double Pr, double Sc,
-                              const Geom& G, cudaStream_t st) {
+                              const Geom& G, int dims, cudaStream_t st) {
     if (Ns == 1)
-        LAUNCH((k_fluxes<F, true, false, true>), cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G, nullptr, nullptr);
+        LAUNCH_FLUXES(F, true, false, true, false, cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G,
+                      nullptr, nullptr);
     else if (pc.eos == CLES_EOS_NASA9)
-        LAUNCH((k_fluxes<F, false, true, true>), cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G, nullptr, nullptr);
+        LAUNCH_FLUXES(F, false, true, true, false, cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G,
+                      nullptr, nullptr);
     else
-        LAUNCH((k_fluxes<F, false, false, true>), cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G, nullptr, nullptr);
+        LAUNCH_FLUXES(F, false, false, true, false, cells, st, Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G,
+                      nullptr, nullptr);
 }
 template <typename F>
 void Pointwise<F>::body_forces(F* dQ, const double* Q, int64_t cells, int Ns, const BodyForces& bf, cudaStream_t st) {
@@ -1352,16 +1223,20 @@ void Pointwise<F>::lsrk(double* Q, double* du, const F* dQ, int64_t n, double A,
     LAUNCH(k_lsrk<F>, n, st, Q, du, dQ, n, A, B, dt, dtp);
 }
 template <typename F>
-void Pointwise<F>::rate(const double* Q, const F* prim, const F* art, double* part, double* out, int64_t cells, int Ns,
-                        const double idx[3], const int act[3], double mu0, double Pr, double Sc, cudaStream_t st) {
-    const unsigned nb = grid_for(cells);
-    k_rate_partial<F><<<nb, kThreads, 0, st>>>(Q, prim, art, part, cells, Ns, idx[0], idx[1], idx[2], act[0], act[1],
-                                               act[2], mu0, Pr, Sc);
+void Pointwise<F>::primitives_rate(const double* Q, F* prim, const F* art, double* part, double* out, int64_t cells,
+                                   int Ns, const PhysConst& pc, const double idx[3], const int act[3], double mu0,
+                                   double Pr, double Sc, cudaStream_t st, int esens) {
+    const RateConst R{{idx[0], idx[1], idx[2]}, {act[0], act[1], act[2]}, mu0, mu0 / Pr, mu0 / Sc};
+    const unsigned nb = (unsigned)rate_partials(cells);
+    if (pc.eos == CLES_EOS_NASA9)
+        k_primitives<F, true, false, true><<<nb, kThreads, 0, st>>>(Q, prim, cells, Ns, pc, esens, nullptr, nullptr, art,
+                                                                    part, R);
+    else
+        k_primitives<F, false, false, true><<<nb, kThreads, 0, st>>>(Q, prim, cells, Ns, pc, esens, nullptr, nullptr,
+                                                                     art, part, R);
     count_launch();
-    check_launch("k_rate_partial");
-    k_rate_final<<<1, kThreads, 0, st>>>(part, (int)nb, out);
-    count_launch();
-    check_launch("k_rate_final");
+    check_launch("k_primitives");
+    rate_final(part, (int)nb, out, st);
 }
 void rate_final(const double* part, int nb, double* out, cudaStream_t st) {
     k_rate_final<<<1, kThreads, 0, st>>>(part, nb, out);
@@ -1389,10 +1264,6 @@ void Pointwise<F>::dissipation(const F* prim, const F* g, const F* art, double* 
     k_sum_final<<<1, kThreads, 0, st>>>(part, (int)nb, 2, out);
     count_launch();
     check_launch("k_sum_final");
-}
-template <typename F>
-void Pointwise<F>::convert(const double* a, F* b, int64_t n, cudaStream_t st) {
-    LAUNCH(k_convert<F>, n, st, a, b, n);
 }
 template <typename F>
 void Pointwise<F>::to_double(const F* a, double* b, int64_t n, cudaStream_t st) {
@@ -1433,7 +1304,14 @@ void gather_interior(const double* padded, double* interior, const int n[3], con
     check_launch("k_gather_interior");
 }
 
-int64_t rate_partials(int64_t cells) { return (int64_t)grid_for(cells); }
+int64_t max_partials(int64_t cells) { return (int64_t)grid_for(cells); }
+
+// Blocks (partials) of a rate reduction: eight per SM, so that the one block of
+// k_rate_final has a few loads a thread (24 us over 9472 partials).
+int64_t rate_partials(int64_t cells) {
+    const int64_t b = (cells + kThreads - 1) / kThreads, most = 8 * (int64_t)num_sms();
+    return std::max<int64_t>(1, std::min(b, most));
+}
 
 template struct Pointwise<double>;
 template struct Pointwise<float>;

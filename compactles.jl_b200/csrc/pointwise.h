@@ -104,42 +104,53 @@ struct BodyForces {
     double g[CLES_MAX_BODY_FORCES][3];
 };
 
+// Fields of one delta4_sum! launch: field k is weighted by h_d^p[k] per dimension.
+template <typename F>
+struct D4Set {
+    const F* in[CLES_MAX_SPECIES + 2];
+    F* out[CLES_MAX_SPECIES + 2];
+    int p[CLES_MAX_SPECIES + 2];
+    int n = 0;
+    void add(const F* i, F* o, int pw) {
+        in[n] = i;
+        out[n] = o;
+        p[n++] = pw;
+    }
+};
+
 template <typename F>
 struct Pointwise {
     // esens: also write the kappa*-sensor input (internal energy) into slot P_Y0 + Ns
     static void primitives(const double* Q, F* prim, int64_t cells, int Ns, const PhysConst& pc, cudaStream_t st,
                            int esens = 0);
-    // delta4_sum! of one (f1 == nullptr) or two fields in one tiled pass
-    static void delta4_tiled(const F* f0, const F* f1, F* o0, F* o1, const Grid3& g, const double w0[3],
-                             const double w1[3], cudaStream_t st);
+    // delta4_sum! of every field of the set in one launch; h: grid spacing
+    static void delta4(const D4Set<F>& fs, const Grid3& g, const double h[3], cudaStream_t st);
     // the same on a rank's block of a decomposed grid: g.periodic is 0 along
     // split dimensions, whose open ends read the exchanged planes of h
     static void delta4_halo(const F* f0, const F* f1, F* o0, F* o1, const Grid3& g, const double w0[3],
                             const double w1[3], const Halo4& h, cudaStream_t st);
-    static void art_coef(const F* s_strain, const F* s_energy, const F* prim, const F* g, F* art, int64_t cells,
-                         double C_mu, double C_beta, double C_kappa, int gate, cudaStream_t st);
-    static void strain(const F* g, F* out, int64_t cells, cudaStream_t st);
-    static void delta4(const F* f, F* out, const Grid3& g, const double wd[3], cudaStream_t st);
-    static void mu_beta(const F* sensor, const F* prim, const F* g, F* art, int64_t cells, double C_mu, double C_beta,
-                        int gate, cudaStream_t st);
+    // sens: the smoothed sensors (strain, internal energy, Y_k when Ns > 1), cells apart
+    static void art_coef(const F* sens, const F* prim, const F* g, F* art, int64_t cells, int Ns, double C_mu,
+                         double C_beta, double C_kappa, double C_D, int gate, cudaStream_t st);
+    // dims: bit d set for an active dimension d, here and in fluxes
+    static void strain(const F* g, F* out, int64_t cells, int dims, cudaStream_t st);
     static void dilatation(const F* g, F* div, F* sw, int64_t cells, cudaStream_t st);
     static void beta_dilatation(const F* sensor, const F* prim, const F* sw, F* art, int64_t cells, double C_beta,
                                 cudaStream_t st);
-    static void energy(const double* Q, const F* prim, F* out, int64_t cells, int Ns, cudaStream_t st);
-    static void kappa(const F* sensor, const F* prim, F* art, int64_t cells, double C_kappa, cudaStream_t st);
-    static void dart(const F* sensor, const F* prim, F* art, int64_t cells, double C_D, int sp, cudaStream_t st);
     static void fluxes(const double* Q, const F* prim, const F* g, const F* gty, const F* art, F* flux, int64_t cells,
-                       int Ns, const PhysConst& pc, double mu0, double Pr, double Sc, cudaStream_t st);
+                       int Ns, const PhysConst& pc, double mu0, double Pr, double Sc, int dims, cudaStream_t st);
     static void lsrk(double* Q, double* du, const F* dQ, int64_t n, double A, double B, double dt, cudaStream_t st,
                      const double* dtp = nullptr);
-    static void rate(const double* Q, const F* prim, const F* art, double* part, double* out, int64_t cells, int Ns,
-                     const double idx[3], const int act[3], double mu0, double Pr, double Sc, cudaStream_t st);
+    // primitives and the max_rate reduction over them (art: the artificial
+    // properties of the last right-hand side) into out = (rate, min density)
+    static void primitives_rate(const double* Q, F* prim, const F* art, double* part, double* out, int64_t cells, int Ns,
+                                const PhysConst& pc, const double idx[3], const int act[3], double mu0, double Pr,
+                                double Sc, cudaStream_t st, int esens);
     static void kinetic(const double* Q, double* part, double* out, int64_t cells, int Ns, cudaStream_t st);
     // G: geometry of a curvilinear / stretched grid (null = unit Jacobian);
     // foldmask bit 2d + side marks a folded edge (quadrature weight 1)
     static void dissipation(const F* prim, const F* g, const F* art, double* part, double* out, const Grid3& gr,
                             double mu0, cudaStream_t st, const Geom* G = nullptr, unsigned foldmask = 0u);
-    static void convert(const double* a, F* b, int64_t n, cudaStream_t st);
     static void to_double(const F* a, double* b, int64_t n, cudaStream_t st);
     // correct_rhs! of an NSCBC face (src/nscbc.jl:59-307) on the plane of
     // (d, side): dpd = dp/dx_d, dpt0/dpt1 = dp along the two transverse dims
@@ -156,7 +167,7 @@ struct Pointwise {
     // (the A_d F_d product of src/rhs.jl:670-675), for curvilinear / stretched grids
     static void fluxes_geo(const double* Q, const F* prim, const F* g, const F* gty, const F* art, F* flux,
                            int64_t cells, int Ns, const PhysConst& pc, double mu0, double Pr, double Sc,
-                           const Geom& G, cudaStream_t st);
+                           const Geom& G, int dims, cudaStream_t st);
 };
 
 // Curvilinear / stretched-grid passes (geometry.cu).
@@ -247,7 +258,8 @@ struct ClockConst {
 };
 void clock_before(double* clk, const double* rate_rmin, const ClockConst& c, cudaStream_t st);
 void clock_after(double* clk, const ClockConst& c, cudaStream_t st);
-int64_t rate_partials(int64_t cells);
+int64_t rate_partials(int64_t cells);   // blocks of a rate reduction
+int64_t max_partials(int64_t cells);    // of any reduction (kinetic energy, dissipation)
 
 // ---- many grids advanced together (batch.cpp) ------------------------------
 // The fields of every grid of a batch live in shared arena blocks: field f of
@@ -263,7 +275,7 @@ struct BatchGrid {
     ClockConst cc;
 };
 // cells of one delta4_sum! tile (x, y, z)
-constexpr int kD4X = 32, kD4Y = 16, kD4Z = 32;
+constexpr int kD4X = 32, kD4Y = 16, kD4Z = 16;
 struct BatchTile { int grid, x0, y0, z0; };     // one delta4 tile (kD4X x kD4Y x kD4Z cells)
 struct BatchFace { int grid, d, side, kind; BcState st; };
 struct BatchChunk { int grid; int64_t c0; };    // cells [c0, c0 + kBatchChunk) of a grid
@@ -276,12 +288,10 @@ struct BatchOps {
     static void primitives(const double* Q, F* prim, int64_t cells_total, int Ns, const PhysConst& pc, int esens,
                            const double* mc, const int* tmap, cudaStream_t st);
     static void fluxes(const double* Q, const F* prim, const F* g, const F* gty, const F* art, F* flux,
-                       int64_t cells_total, int Ns, const PhysConst& pc, double mu0, double Pr, double Sc,
+                       int64_t cells_total, int Ns, const PhysConst& pc, double mu0, double Pr, double Sc, int dims,
                        const double* mc, const int* tmap, cudaStream_t st);
-    // delta4_sum! of one (f1 == nullptr) or two fields of every grid; field k
-    // is weighted by h_d^pk per dimension
-    static void delta4(const F* f0, const F* f1, F* o0, F* o1, int p0, int p1, const BatchGrid* grids,
-                       const BatchTile* tiles, int ntiles, int64_t cells_total, cudaStream_t st);
+    // delta4_sum! of the set's fields (block starts) on every grid
+    static void delta4(const D4Set<F>& fs, const BatchGrid* grids, const BatchTile* tiles, int ntiles, cudaStream_t st);
     // max_rate of every grid (per-chunk partials, then one block per grid
     // reduces them) followed by the graph-mode clock_before of that grid;
     // chunk_first[g] .. chunk_first[g + 1] are grid g's chunks

@@ -69,6 +69,9 @@ inline double jmin(double x, double y) {
     return y < x ? y : x;
 }
 
+// scratch fields: the strain, the smoothed sensors, at least five
+inline int n_scratch(int Ns) { return std::max(5, 3 + Ns); }
+
 template <typename F>
 class Solver final : public SolverBase {
 public:
@@ -170,9 +173,9 @@ public:
         g_u_.alloc(ctx, sizeof(F) * c * 9);
         gty_.alloc(ctx, sizeof(F) * c * 3 * (1 + Ns_));
         art_.alloc(ctx, sizeof(F) * c * (A_D0 + Ns_));
-        scratch_.alloc(ctx, sizeof(F) * c * 5);
+        scratch_.alloc(ctx, sizeof(F) * c * n_scratch(Ns_));
         flux_.alloc(ctx, sizeof(F) * c * 3 * ncons_);
-        part_.alloc(ctx, sizeof(double) * 2 * (size_t)(rate_partials(cells_) + 1));
+        part_.alloc(ctx, sizeof(double) * 2 * (size_t)(max_partials(cells_) + 1));
         res_.alloc(ctx, sizeof(double) * 4);
         CLES_CUDA(cudaMallocHost(&host_res_, sizeof(double) * 4));
         // du, gradients of collapsed dims and the artificial properties start
@@ -342,14 +345,23 @@ public:
         throw Error(CLES_EINVAL, "internal: no split plan for this operator");
     }
 
-    // delta4_sum! of one or two fields (src/artificial.jl:67-94); on a
-    // decomposed grid the two planes beyond each rank interface of every split
-    // dim are exchanged first (the reference's exchange_halos! before it).
-    void delta4(const F* f0, const F* f1, F* o0, F* o1, const double w0[3], const double w1[3]) {
+    // delta4_sum! of the set's fields (src/artificial.jl:67-94); on a decomposed
+    // grid two fields at a time, the two planes beyond each rank interface of
+    // every split dim exchanged first (the reference's exchange_halos! before it).
+    void delta4(const D4Set<F>& fs) {
         if (!decomposed_) {
-            Pointwise<F>::delta4_tiled(f0, f1, o0, o1, g_, w0, w1, st_);
+            Pointwise<F>::delta4(fs, g_, h_, st_);
             return;
         }
+        double w[2][3];
+        for (int f = 0; f < fs.n; f += 2) {
+            const bool two = f + 1 < fs.n;
+            for (int e = 0; e < (two ? 2 : 1); ++e)
+                for (int k = 0; k < 3; ++k) w[e][k] = fs.p[f + e] == 2 ? h_[k] * h_[k] : h_[k];
+            delta4_split(fs.in[f], two ? fs.in[f + 1] : nullptr, fs.out[f], two ? fs.out[f + 1] : nullptr, w[0], w[1]);
+        }
+    }
+    void delta4_split(const F* f0, const F* f1, F* o0, F* o1, const double w0[3], const double w1[3]) {
         Halo4 h{};
         Grid3 gl = g_;
         const int dt = sizeof(F) == 8 ? CLES_F64 : CLES_F32;
@@ -658,6 +670,8 @@ public:
     // ------------------------------------------------------------- views --
     FieldView view(void* p) const { return FieldView{p, cells_, g_.n[0], (int64_t)g_.n[0] * g_.n[1]}; }
     F* prim(int slot) const { return prim_.as<F>() + (size_t)cells_ * slot; }
+    // bit d: dimension d is resolved
+    int dims() const { return (g_.active[0] ? 1 : 0) | (g_.active[1] ? 2 : 0) | (g_.active[2] ? 4 : 0); }
     F* scratch(int k) const { return scratch_.as<F>() + (size_t)cells_ * k; }
 
     // --------------------------------------------------------- operators --
@@ -825,37 +839,35 @@ public:
     }
 
     void compute_artificial() {
-        // compute_artificial! (src/artificial.jl:261-359).  The strain and the
-        // internal-energy sensor chains are independent, so their fourth
-        // differences are one tiled pass, their smoothing one batched filter
-        // launch per direction, and mu*, beta*, kappa* one pointwise pass; each
-        // field sees the reference's operations in the reference's order.
+        // compute_artificial! (src/artificial.jl:261-359).  The sensor chains
+        // (strain, internal energy and, with several species, the mass fractions)
+        // are independent: one delta4 launch, one batched filter launch per
+        // direction and one pass for all coefficients; each field sees the
+        // reference's operations in the reference's order.
         if (!desc.art_enabled) return;
         using PW = Pointwise<F>;
         F* strain = scratch(0);
-        F* sensor = scratch(1);     // smoothed strain sensor
-        F* sensor_e = scratch(2);   // smoothed internal-energy sensor (adjacent: batched smoothing)
-        F* tmp_a = scratch(3);
-        F* tmp_b = scratch(4);
-        const double w2[3] = {h_[0] * h_[0], h_[1] * h_[1], h_[2] * h_[2]};
-        const double w1[3] = {h_[0], h_[1], h_[2]};
-        PW::strain(g_u_.as<F>(), strain, cells_, st_);
-        delta4(strain, prim(P_Y0 + Ns_), sensor, sensor_e, w2, w1);
-        smooth(sensor, 2);
-        PW::art_coef(sensor, sensor_e, prim_.as<F>(), g_u_.as<F>(), art_.as<F>(), cells_, desc.C_mu, desc.C_beta,
-                     desc.C_kappa, desc.beta_sensor == CLES_BETA_GATED_STRAIN, st_);
+        F* sensors = scratch(1);    // smoothed: strain, internal energy (get_field's sensor), Y_k
+        const int ns = Ns_ > 1 ? 2 + Ns_ : 2;
+        // curvature terms fill the collapsed dimensions' gradients on curvilinear grids
+        PW::strain(g_u_.as<F>(), strain, cells_, geo_ ? 7 : dims(), st_);
+        D4Set<F> fs;
+        fs.add(strain, sensors, 2);
+        fs.add(prim(P_Y0 + Ns_), scratch(2), 1);
+        for (int sp = 0; sp < ns - 2; ++sp) fs.add(prim(P_Y0 + sp), scratch(3 + sp), 1);
+        delta4(fs);
+        smooth(sensors, ns);
+        PW::art_coef(sensors, prim_.as<F>(), g_u_.as<F>(), art_.as<F>(), cells_, Ns_, desc.C_mu, desc.C_beta,
+                     desc.C_kappa, desc.C_D, desc.beta_sensor == CLES_BETA_GATED_STRAIN, st_);
         if (desc.beta_sensor == CLES_BETA_DILATATION) {
+            F* tmp_a = scratch(3);
+            F* tmp_b = scratch(4);
             PW::dilatation(g_u_.as<F>(), tmp_a, tmp_b, cells_, st_);
-            delta4(tmp_a, nullptr, sensor, nullptr, w2, w2);
-            smooth(sensor, 1);
-            PW::beta_dilatation(sensor, prim_.as<F>(), tmp_b, art_.as<F>(), cells_, desc.C_beta, st_);
-        }
-        if (Ns_ > 1) {
-            for (int sp = 0; sp < Ns_; ++sp) {
-                delta4(prim(P_Y0 + sp), nullptr, tmp_a, nullptr, w1, w1);
-                smooth(tmp_a, 1);
-                PW::dart(tmp_a, prim_.as<F>(), art_.as<F>(), cells_, desc.C_D, sp, st_);
-            }
+            D4Set<F> fd;
+            fd.add(tmp_a, sensors, 2);
+            delta4(fd);
+            smooth(sensors, 1);
+            PW::beta_dilatation(sensors, prim_.as<F>(), tmp_b, art_.as<F>(), cells_, desc.C_beta, st_);
         }
     }
 
@@ -880,7 +892,7 @@ public:
         if (geo_) {
             MetricOps<F>::scale_grad(gty_.as<F>(), ngty, G_, g_, st_);
             PW::fluxes_geo(Q_.as<double>(), prim_.as<F>(), g_u_.as<F>(), gty_.as<F>(), art_.as<F>(), flux_.as<F>(),
-                           cells_, Ns_, pc_, desc.mu0, desc.Pr, desc.Sc, G_, st_);
+                           cells_, Ns_, pc_, desc.mu0, desc.Pr, desc.Sc, G_, dims(), st_);
             // general path (src/rhs.jl:669-687): D_d(A_d F_d) in place over the
             // flux block, then dQ = -sum_d inv_J D_d(A_d F_d) + metric sources
             for (int k = 0; k < 3; ++k) {
@@ -895,7 +907,7 @@ public:
             return false;
         }
         PW::fluxes(Q_.as<double>(), prim_.as<F>(), g_u_.as<F>(), gty_.as<F>(), art_.as<F>(), flux_.as<F>(), cells_, Ns_,
-                   pc_, desc.mu0, desc.Pr, desc.Sc, st_);
+                   pc_, desc.mu0, desc.Pr, desc.Sc, dims(), st_);
         // flux divergence dQ[c] = -sum_d D_d(F_dc) (src/rhs.jl:650-668), accumulated in the store.
         // With all three dims active the order is y, x, z: the first direction only
         // stores (no read of dQ), the x kernel reads dQ with vector loads, and z,
@@ -976,9 +988,10 @@ public:
         if (geo_) MetricOps<F>::metric_grad(g_u_.as<F>(), prim_.as<F>(), G_, g_, st_);
     }
 
-    // the rate reduction of max_rate on the refreshed primitives
-    void rate_pass() {
+    // the primitives of the resident state and the rate reduction of max_rate over them
+    void primitives_rate() {
         if (geo_) {
+            Pointwise<F>::primitives(Q_.as<double>(), prim_.as<F>(), cells_, Ns_, pc_, st_, desc.art_enabled);
             MetricOps<F>::rate_geo(Q_.as<double>(), prim_.as<F>(), art_.as<F>(), part_.as<double>(), res_.as<double>(),
                                    Ns_, h_, desc.mu0, desc.Pr, desc.Sc, G_, g_, st_);
             return;
@@ -986,13 +999,13 @@ public:
         double idx[3];
         int act[3];
         for (int k = 0; k < 3; ++k) { idx[k] = 1.0 / h_[k]; act[k] = g_.active[k]; }
-        Pointwise<F>::rate(Q_.as<double>(), prim_.as<F>(), art_.as<F>(), part_.as<double>(), res_.as<double>(), cells_,
-                           Ns_, idx, act, desc.mu0, desc.Pr, desc.Sc, st_);
+        Pointwise<F>::primitives_rate(Q_.as<double>(), prim_.as<F>(), art_.as<F>(), part_.as<double>(),
+                                      res_.as<double>(), cells_, Ns_, pc_, idx, act, desc.mu0, desc.Pr, desc.Sc, st_,
+                                      desc.art_enabled);
     }
 
     void max_rate(double* rate, double* rho_min) override {
-        Pointwise<F>::primitives(Q_.as<double>(), prim_.as<F>(), cells_, Ns_, pc_, st_, desc.art_enabled);
-        rate_pass();
+        primitives_rate();
         CLES_CUDA(cudaMemcpyAsync(host_res_, res_.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, st_));
         CLES_CUDA(cudaStreamSynchronize(st_));
         if (take_device_timeouts(st_))
@@ -1206,8 +1219,7 @@ public:
         try {
             double* clk = clk_.as<double>();
             apply_bcs();
-            Pointwise<F>::primitives(Q_.as<double>(), prim_.as<F>(), cells_, Ns_, pc_, st_, desc.art_enabled);
-            rate_pass();
+            primitives_rate();
             clock_before(clk, res_.as<double>(), cc_, st_);
             for (int stage = 0; stage < 5; ++stage) {
                 if (stage > 0) apply_bcs();
@@ -1444,7 +1456,7 @@ size_t solver_bytes_estimate(const cles_solver_desc& d) {
     const int Ns = d.n_species, nc = Ns + 4;
     const size_t F = d.precision == CLES_PREC_MIXED ? sizeof(float) : sizeof(double);
     const size_t per_cell = 2 * nc * sizeof(double)                     // Q, du
-                            + F * (nc + (P_Y0 + Ns + 1) + 9 + 3 * (1 + Ns) + (A_D0 + Ns) + 5 + 3 * nc) +
+                            + F * (nc + (P_Y0 + Ns + 1) + 9 + 3 * (1 + Ns) + (A_D0 + Ns) + n_scratch(Ns) + 3 * nc) +
                             (d.control.retries > 0 ? nc * sizeof(double) : 0);
     return (size_t)cells * per_cell + ((size_t)4 << 20);  // + plan tables and reduction scratch
 }
