@@ -773,7 +773,9 @@ private:
     // streams between a fork and a join on the batch stream.  OUT_RK tries the
     // fused update; a member whose kernel cannot fuse it gets a subtracting
     // store, and its `rk_fused_` entry says so for the separate RK pass.
-    void along_members(int role, int k, const void* in, void* out, int count, int mode, int stage) {
+    // in2 / out2 / count2: a second group of fields under the same operator.
+    void along_members(int role, int k, const void* in, void* out, int count, int mode, int stage,
+                       const void* in2 = nullptr, void* out2 = nullptr, int count2 = 0) {
         const size_t el = (role == R_QFILT || sizeof(F) == 8) ? sizeof(double) : sizeof(float);
         CLES_CUDA(cudaEventRecord(fork_ev_, st_));
         const int ns = std::min<int>(kAuxStreams, (int)order_.size());
@@ -791,6 +793,10 @@ private:
                 const bool fused = launch_compact_rk(*p, vin, vout, count, rk, st);
                 if (!fused) launch_compact(*p, vin, vout, count, OUT_SUBTRACT, st);
                 rk_fused_[g] = fused ? 1 : 0;
+            } else if (count2 > 0) {
+                const FieldView vin2{const_cast<char*>(static_cast<const char*>(in2)) + el * (size_t)m.off, ct_, sy, sz};
+                const FieldView vout2{static_cast<char*>(out2) + el * (size_t)m.off, ct_, sy, sz};
+                launch_compact_pair(*p, vin, vout, count, vin2, vout2, count2, st);
             } else {
                 launch_compact(*p, vin, vout, count, mode, st);
             }
@@ -858,12 +864,21 @@ private:
     void rhs_and_update(bool primitives_current, int stage) {
         using PW = Pointwise<F>;
         if (!primitives_current) primitives();
-        for (int k = 0; k < 3; ++k)
-            if (act_[k]) along(R_DERIV, k, field(prim_, P_U), g_u_.as<F>() + (size_t)ct_ * 3 * k, 3, OUT_STORE);
-        artificial();
         const int ngty = Ns_ == 1 ? 1 : 1 + Ns_;
         for (int k = 0; k < 3; ++k)
-            if (act_[k]) along(R_DERIV, k, field(prim_, P_T), gty_.as<F>() + (size_t)ct_ * ngty * k, ngty, OUT_STORE);
+            if (act_[k]) {
+                // velocity, temperature and mass-fraction gradients: per-member
+                // kernels take both groups in one launch
+                F* g = g_u_.as<F>() + (size_t)ct_ * 3 * k;
+                F* gt = gty_.as<F>() + (size_t)ct_ * ngty * k;
+                if (roles_[R_DERIV][k].per_member) {
+                    along_members(R_DERIV, k, field(prim_, P_U), g, 3, OUT_STORE, 0, field(prim_, P_T), gt, ngty);
+                } else {
+                    along(R_DERIV, k, field(prim_, P_U), g, 3, OUT_STORE);
+                    along(R_DERIV, k, field(prim_, P_T), gt, ngty, OUT_STORE);
+                }
+            }
+        artificial();
         BatchOps<F>::fluxes(Q_.as<double>(), prim_.as<F>(), g_u_.as<F>(), gty_.as<F>(), art_.as<F>(), flux_.as<F>(),
                             ct_, Ns_, pc_, cls_.mu0, cls_.Pr, cls_.Sc, dims(), mc_.as<double>(), tmap_.as<int>(), st_);
         // dQ = -sum_d D_d(F_d) with the RK update in the last direction's store

@@ -139,6 +139,15 @@ struct LineCoef {
     T ci[CLES_MAX_M], a0, pad_;
 };
 
+// Where element e (of n: [2q rows][Wn segments][2q end values]) of segment s's
+// inverse rows sits.  Short tiles run few lines a block, so that the lanes of a
+// warp hold neighbouring segments: segment fastest.  The others share a segment
+// among 16 or 32 lanes: a segment's elements together, for wide broadcast loads
+// (C10 on 201x161x129: 254 us against 299 us segment-fastest).
+__host__ __device__ inline size_t line_row_index(int MS, int S, int n, int e, int s) {
+    return MS == 16 ? (size_t)e * S + s : (size_t)s * n + e;
+}
+
 // Segmented form of a line of any length (k_line): S segments, the first `rem`
 // of base + 1 points and the others of base, on register tiles of MS points.
 struct LinePlan {
@@ -146,16 +155,21 @@ struct LinePlan {
     int mm = 0;                       // longest segment, rounded up to a group of four rows
     int Wn = 0, Kr = 0;               // interface window: segments, radius
     std::vector<unsigned char> coef;  // LineCoef<plan dtype, q, MS>
-    std::vector<unsigned char> host_tab;   // reduced inverse rows, [S][2q][Wn][2q], until they are on the device
+    std::vector<unsigned char> host_tab;   // reduced inverse rows (line_row_index), until they are on the device
     const void* dcoef = nullptr;      // coef and those rows in the plan's device block
     const void* tab = nullptr;
 };
 struct LineArgs {
     FieldView in, out;
+    // fields split .. are fields 0 .. of a second group under the same operator
+    // (strides of the first)
+    const void* in2;
+    void* out2;
+    int split;
     int S, base, rem, mm, Wn, Kr;
     int logL, SC, CL;                 // lines (log2) and segments per block, blocks per cluster
     int pitch, kpad;                  // shared row of an x line: pitch, one pad element every 2^kpad
-    int gstage;                       // the block's inverse rows are staged in shared memory
+    int gstage;                       // the inverse rows are staged in shared memory
     int mode, rk_first;
     struct {
         double *Q, *du;
@@ -229,8 +243,14 @@ bool try_launch_xt(const CompactPlan& plan, const FieldView& in, const FieldView
 // k_line launch; false (and nothing launched) when the plan has no line form.
 // rk: the RK update of mode OUT_RK; rk_first: no earlier direction stored into
 // `out`, the divergence is this direction's alone.
+// in2 / out2 / count2: a second group of fields, views of the same strides.
 bool try_launch_line(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
-                     cudaStream_t st, const RkEpilogue* rk = nullptr, bool rk_first = false);
+                     cudaStream_t st, const RkEpilogue* rk = nullptr, bool rk_first = false,
+                     const void* in2 = nullptr, void* out2 = nullptr, int count2 = 0);
+// The operator over two groups of fields (OUT_STORE, views of the same strides):
+// one launch where the kernel can take both, else two.
+void launch_compact_pair(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count,
+                         const FieldView& in2, const FieldView& out2, int count2, cudaStream_t st);
 // Flux divergence of the last direction fused with the RK update; false (and
 // nothing launched) when the plan takes neither the TMA path nor k_line.  first:
 // the only direction, `out` holds nothing yet (and is not written).

@@ -272,12 +272,12 @@ void dispatch(const CompactParams& P, const T* tab, const FieldView& in, const F
 }  // namespace
 
 bool launch_line_f64(const CompactPlan&, const FieldView&, const FieldView&, int, int, cudaStream_t, const RkEpilogue&,
-                     bool, int);
+                     bool, const void*, void*, int, int);
 bool launch_line_f32(const CompactPlan&, const FieldView&, const FieldView&, int, int, cudaStream_t, const RkEpilogue&,
-                     bool, int);
+                     bool, const void*, void*, int, int);
 
 bool try_launch_line(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
-                     cudaStream_t st, const RkEpilogue* rkp, bool rk_first) {
+                     cudaStream_t st, const RkEpilogue* rkp, bool rk_first, const void* in2, void* out2, int count2) {
     if (!plan.line || (mode == OUT_RK && !rkp)) return false;
     // byte offsets along a segment are 32-bit
     const int64_t st_in = plan.P.dim == 0 ? 1 : plan.P.dim == 1 ? in.sy : in.sz;
@@ -285,8 +285,8 @@ bool try_launch_line(const CompactPlan& plan, const FieldView& in, const FieldVi
     if (std::max(st_in, st_out) * 8 * 64 >= (int64_t)1 << 31) return false;
     RkEpilogue rk{nullptr, nullptr, 0.0, 0.0, 0.0, nullptr};
     if (rkp) rk = *rkp;
-    return plan.dtype == CLES_F64 ? launch_line_f64(plan, in, out, count, mode, st, rk, rk_first, num_sms())
-                                  : launch_line_f32(plan, in, out, count, mode, st, rk, rk_first, num_sms());
+    return (plan.dtype == CLES_F64 ? launch_line_f64 : launch_line_f32)(plan, in, out, count, mode, st, rk, rk_first, in2,
+                                                                        out2, count2, num_sms());
 }
 
 // Which kernel a line solve takes.  Periodic tridiagonal x lines of 32 k points:
@@ -321,6 +321,18 @@ void launch_compact(const CompactPlan& plan, const FieldView& in, const FieldVie
         dispatch<float>(plan.P, plan.tab32, in, out, count, mode, st);
     }
     if (rec >= 0) prof_end(rec, st);
+}
+
+void launch_compact_pair(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count,
+                         const FieldView& in2, const FieldView& out2, int count2, cudaStream_t st) {
+    const bool same = in.comp_stride == in2.comp_stride && in.sy == in2.sy && in.sz == in2.sz &&
+                      out.comp_stride == out2.comp_stride && out.sy == out2.sy && out.sz == out2.sz;
+    // (a profiled launch is bracketed by launch_compact)
+    if (same && !profiling() && count > 0 && count2 > 0 && plan.P.lines > 0 && !plan.has_xw && !tile_first(plan) &&
+        try_launch_line(plan, in, out, count, OUT_STORE, st, nullptr, false, in2.base, out2.base, count2))
+        return;
+    launch_compact(plan, in, out, count, OUT_STORE, st);
+    launch_compact(plan, in2, out2, count2, OUT_STORE, st);
 }
 
 bool launch_compact_rk(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count,

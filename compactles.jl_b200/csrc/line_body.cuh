@@ -40,6 +40,9 @@ __device__ __forceinline__ void ln_cp_async(float* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(ln_smem(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void ln_cluster_arrive() { asm volatile("barrier.cluster.arrive;" ::: "memory"); }
+__device__ __forceinline__ void ln_cluster_arrive_relaxed() {
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+}
 __device__ __forceinline__ void ln_cluster_wait() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
 // shared-window address of `addr` in block `rank` of the cluster
 __device__ __forceinline__ unsigned ln_map(unsigned addr, unsigned rank) {
@@ -164,11 +167,11 @@ __device__ __forceinline__ void ln_correct(const K& C, const int mm, T (&y)[MS],
     }
 }
 
-// Registers a thread: two 256-thread blocks per SM in FP64, three in FP32, and
-// as many again with the short tile.
-template <typename T, int MS>
+// Registers a thread: 16 to 24 warps on an SM in FP64, 24 to 32 in FP32 (without
+// spills; the filter's wide stencil takes more).
+template <typename T, int M, int MS>
 constexpr int ln_regs() {
-    return sizeof(T) == 8 ? (MS == 32 ? 128 : MS == 24 ? 112 : 96) : (MS == 32 ? 80 : 64);
+    return sizeof(T) == 8 ? (MS == 32 ? 128 : MS == 24 ? 104 : M <= 2 ? 80 : 96) : (MS == 32 ? 80 : 64);
 }
 
 // Small plans (the short tile) run in a few microseconds, which straight-line
@@ -199,7 +202,7 @@ __device__ __forceinline__ void ln_stage(T* dst, const T* src, int count) {
 }
 
 template <typename T, int Q, int M, int MS, bool XM>
-__global__ void __maxnreg__((ln_regs<T, MS>())) k_line(const __grid_constant__ CompactParams P,
+__global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant__ CompactParams P,
                                                        const __grid_constant__ LnParam<T, Q, MS> C,
                                                        const __grid_constant__ LineArgs A, const T* __restrict__ Gw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -222,17 +225,18 @@ __global__ void __maxnreg__((ln_regs<T, MS>())) k_line(const __grid_constant__ C
     const int m = base + (seg < A.rem ? 1 : 0);
     const int mm = A.mm;
     const bool periodic = P.periodic != 0;
-    const T* fin = reinterpret_cast<const T*>(A.in.base) + (int64_t)comp * A.in.comp_stride;
-    T* fout = reinterpret_cast<T*>(A.out.base) + (int64_t)comp * A.out.comp_stride;
+    const bool second = comp >= A.split;
+    const int fc = second ? comp - A.split : comp;
+    const T* fin = static_cast<const T*>(second ? A.in2 : A.in.base) + (int64_t)fc * A.in.comp_stride;
+    T* fout = static_cast<T*>(second ? A.out2 : A.out.base) + (int64_t)fc * A.out.comp_stride;
     T* tile = reinterpret_cast<T*>(smem_raw);
     T* ht = XM ? tile + (size_t)L * A.pitch : tile;   // [SC][2q][L]
-    // shared copies of a small plan: coefficients, inverse rows of the block's segments
+    // shared copies of a small plan: coefficients, inverse rows
     T* csm = ht + (size_t)SC * 2 * Q * L;
-    const int grow = 2 * Q * A.Wn * 2 * Q;   // elements of a segment's inverse rows
     T* gsm = csm + sizeof(Coef) / sizeof(T);
     if constexpr (CS) {
         ln_stage(csm, reinterpret_cast<const T*>(C), (int)(sizeof(Coef) / sizeof(T)));
-        if (A.gstage) ln_stage(gsm, Gw + (int64_t)seg0 * grow, min(SC, S - seg0) * grow);
+        if (A.gstage) ln_stage(gsm, Gw, 2 * Q * A.Wn * 2 * Q * S);
     }
 
     // element offset of point 0 of x line l
@@ -430,7 +434,9 @@ __global__ void __maxnreg__((ln_regs<T, MS>())) k_line(const __grid_constant__ C
         for (int t = 0; t < Q; ++t) ap[t] = an[t] = T(0);
         if (ok) {
             const int Wn = A.Wn;
-            const T* g = CS && A.gstage ? gsm + sl * grow : Gw + (int64_t)seg * grow;
+            // this segment's rows (line_row_index)
+            const T* g = CS ? (A.gstage ? gsm : Gw) + seg : Gw + (int64_t)seg * (2 * Q) * Wn * (2 * Q);
+            const int ge = CS ? S : 1;
             // first segments of the two windows (around seg - 1 and seg + 1)
             int jp = seg - 1 - A.Kr, jn = seg + 1 - A.Kr;
             if (periodic) {
@@ -442,6 +448,7 @@ __global__ void __maxnreg__((ln_regs<T, MS>())) k_line(const __grid_constant__ C
                 jn = max(0, min(jn, S - Wn));
             }
             if (CL == 1) {
+#pragma unroll(CS ? 3 : 1)
                 for (int j = 0; j < Wn; ++j) {
 #pragma unroll
                     for (int u = 0; u < 2 * Q; ++u) {
@@ -449,8 +456,8 @@ __global__ void __maxnreg__((ln_regs<T, MS>())) k_line(const __grid_constant__ C
                         const T hn = ht[(size_t)(jn * 2 * Q + u) * L + lane];
 #pragma unroll
                         for (int t = 0; t < Q; ++t) {
-                            ap[t] += g[(t * Wn + j) * 2 * Q + u] * hp;
-                            an[t] += g[((Q + t) * Wn + j) * 2 * Q + u] * hn;
+                            ap[t] += g[((t * Wn + j) * 2 * Q + u) * ge] * hp;
+                            an[t] += g[(((Q + t) * Wn + j) * 2 * Q + u) * ge] * hn;
                         }
                     }
                     jp = jp + 1 == S ? 0 : jp + 1;
@@ -459,6 +466,7 @@ __global__ void __maxnreg__((ln_regs<T, MS>())) k_line(const __grid_constant__ C
             } else {
                 const unsigned hb = ln_smem(ht) + (unsigned)(lane * sizeof(T));
                 const unsigned rowb = (unsigned)(L * sizeof(T));
+#pragma unroll(CS ? 3 : 1)
                 for (int j = 0; j < Wn; ++j) {
                     const int cp = jp / SC, cn = jn / SC;
                     const unsigned bp = ln_map(hb, cp) + (unsigned)((jp - cp * SC) * 2 * Q) * rowb;
@@ -469,8 +477,8 @@ __global__ void __maxnreg__((ln_regs<T, MS>())) k_line(const __grid_constant__ C
                         const T hn = ln_remote(bn + u * rowb, T(0));
 #pragma unroll
                         for (int t = 0; t < Q; ++t) {
-                            ap[t] += g[(t * Wn + j) * 2 * Q + u] * hp;
-                            an[t] += g[((Q + t) * Wn + j) * 2 * Q + u] * hn;
+                            ap[t] += g[((t * Wn + j) * 2 * Q + u) * ge] * hp;
+                            an[t] += g[(((Q + t) * Wn + j) * 2 * Q + u) * ge] * hn;
                         }
                     }
                     jp = jp + 1 == S ? 0 : jp + 1;
@@ -484,8 +492,9 @@ __global__ void __maxnreg__((ln_regs<T, MS>())) k_line(const __grid_constant__ C
             zn[t] = an[t];
         }
     }
-    // no block leaves while another may still read its end values
-    if (CL > 1) ln_cluster_arrive();
+    // no block leaves while another may still read its end values (nothing to
+    // publish: a relaxed arrival)
+    if (CL > 1) ln_cluster_arrive_relaxed();
     if constexpr (CS) {
         ln_correct<T, Q, MS>(LnShared<T, Q, MS>((ln_coef<T, Q, MS>(C, csm)), cls), mm, y, zp, zn);
     } else {
@@ -628,15 +637,17 @@ __global__ void __maxnreg__((ln_regs<T, MS>())) k_line(const __grid_constant__ C
     if (CL > 1) ln_cluster_wait();
 }
 
-// Lines and segments per block.  Blocks of about 256 threads (two or more per
-// SM at 128 registers); long lines are spread over a cluster of up to 8 blocks.
-// Fewer lines a block where the launch would not fill the SMs twice: down to 8
-// (64-byte rows) along y and z, where lanes are consecutive x, down to 1 along
-// x, where rows are contiguous.
+// Lines and segments per block.  Blocks of at most 256 threads (two or more per
+// SM): 32 lines each, 16 where that keeps a line in one block (x rows are
+// contiguous, and 16 FP64 y / z lanes still fill 128-byte rows; FP32 y / z lines
+// keep 32), else the line over a cluster of up to 8 blocks.  Fewer lines a block
+// where the launch would not fill the SMs twice: down to 8 (64-byte rows) along y
+// and z, 1 along x; and one block of up to 512 threads rather than a cluster where
+// it cannot fill them once.
 struct LineShape {
     int L, SC, CL;
 };
-inline LineShape line_shape(const CompactParams& P, const LinePlan& lp, int count, int num_sms) {
+inline LineShape line_shape(const CompactParams& P, const LinePlan& lp, int count, int num_sms, size_t el) {
     auto shape = [&](int L) {
         LineShape s;
         s.L = L;
@@ -648,25 +659,28 @@ inline LineShape line_shape(const CompactParams& P, const LinePlan& lp, int coun
     };
     const int lmin = P.dim == 0 ? 1 : 8;
     int L = 32;
+    if (lp.S * L > 256 && (P.dim == 0 || el == 8)) L = 16;
     while (L > lmin && L / 2 >= P.lines) L /= 2;
     while (L > 1 && shape(L).SC * L > 512) L /= 2;
     auto blocks = [&](int l) { return ((P.lines + l - 1) / l) * count * shape(l).CL; };
     while (L > lmin && blocks(L) < 2 * num_sms) L /= 2;
     LineShape s = shape(L);
-    // a launch that cannot fill the device anyway: one block rather than a cluster
     if (s.CL > 1 && lp.S * L <= 512 && blocks(L) < num_sms) s = LineShape{L, lp.S, 1};
     return s;
 }
 
 template <typename T, int Q, int M, int MS, bool XM>
 void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
-                   cudaStream_t st, const RkEpilogue& rk, bool rk_first, int num_sms) {
+                   cudaStream_t st, const RkEpilogue& rk, bool rk_first, const void* in2, void* out2, int count2, int num_sms) {
     const CompactParams& P = plan.P;
     const LinePlan& lp = *plan.line;
-    const LineShape s = line_shape(P, lp, count, num_sms);
+    const LineShape s = line_shape(P, lp, count + count2, num_sms, sizeof(T));
     LineArgs A;
     A.in = in;
     A.out = out;
+    A.in2 = in2;
+    A.out2 = out2;
+    A.split = count;
     A.S = lp.S;
     A.base = lp.base;
     A.rem = lp.rem;
@@ -690,8 +704,8 @@ void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView
     A.gstage = 0;
     if (ln_shared<MS>()) {
         smem += sizeof(LineCoef<T, Q, MS>);
-        const size_t g = sizeof(T) * (size_t)s.SC * 2 * Q * lp.Wn * 2 * Q;
-        if (g <= 32 * 1024) {
+        const size_t g = sizeof(T) * (size_t)lp.S * 2 * Q * lp.Wn * 2 * Q;
+        if (g <= 16 * 1024) {
             A.gstage = 1;
             smem += g;
         }
@@ -700,7 +714,7 @@ void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView
     if (smem > 48 * 1024)
         CLES_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((P.lines + s.L - 1) / s.L) * s.CL, (unsigned)count);
+    cfg.gridDim = dim3((unsigned)((P.lines + s.L - 1) / s.L) * s.CL, (unsigned)(count + count2));
     // whole warps for the row copies; threads past SC segments only take part
     // in those and in the barriers
     cfg.blockDim = dim3((unsigned)((s.L * s.SC + 31) / 32 * 32));
@@ -726,20 +740,20 @@ void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView
 
 template <typename T, int Q, int M, bool XM>
 void launch_line_ms(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
-                    cudaStream_t st, const RkEpilogue& rk, bool rk_first, int num_sms) {
-    if (plan.line->MS == 16) launch_line_t<T, Q, M, 16, XM>(plan, in, out, count, mode, st, rk, rk_first, num_sms);
-    else if (plan.line->MS == 24) launch_line_t<T, Q, M, 24, XM>(plan, in, out, count, mode, st, rk, rk_first, num_sms);
-    else launch_line_t<T, Q, M, 32, XM>(plan, in, out, count, mode, st, rk, rk_first, num_sms);
+                    cudaStream_t st, const RkEpilogue& rk, bool rk_first, const void* in2, void* out2, int count2, int num_sms) {
+    if (plan.line->MS == 16) launch_line_t<T, Q, M, 16, XM>(plan, in, out, count, mode, st, rk, rk_first, in2, out2, count2, num_sms);
+    else if (plan.line->MS == 24) launch_line_t<T, Q, M, 24, XM>(plan, in, out, count, mode, st, rk, rk_first, in2, out2, count2, num_sms);
+    else launch_line_t<T, Q, M, 32, XM>(plan, in, out, count, mode, st, rk, rk_first, in2, out2, count2, num_sms);
 }
 
 template <typename T>
 bool launch_line_dtype(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
-                       cudaStream_t st, const RkEpilogue& rk, bool rk_first, int num_sms) {
+                       cudaStream_t st, const RkEpilogue& rk, bool rk_first, const void* in2, void* out2, int count2, int num_sms) {
     const CompactParams& P = plan.P;
     auto go = [&](auto q, auto m) {
         constexpr int Q = decltype(q)::value, M = decltype(m)::value;
-        if (P.dim == 0) launch_line_ms<T, Q, M, true>(plan, in, out, count, mode, st, rk, rk_first, num_sms);
-        else launch_line_ms<T, Q, M, false>(plan, in, out, count, mode, st, rk, rk_first, num_sms);
+        if (P.dim == 0) launch_line_ms<T, Q, M, true>(plan, in, out, count, mode, st, rk, rk_first, in2, out2, count2, num_sms);
+        else launch_line_ms<T, Q, M, false>(plan, in, out, count, mode, st, rk, rk_first, in2, out2, count2, num_sms);
         return true;
     };
     using I1 = std::integral_constant<int, 1>;

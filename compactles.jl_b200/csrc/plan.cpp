@@ -236,9 +236,11 @@ void pack_line_coef(LinePlan& lp, const CompactParams& P, const std::vector<doub
     else pack_line_coef<T, Q, 32>(lp, P, f, v, w, tl);
 }
 
-// Segments of at most MS points: 32 per thread where the plan's points fill
-// the device with them, 16 below that (twice the threads, half the chain).
-constexpr int64_t kLineWide = (int64_t)1 << 21;
+// Segments of at most 32 points; of 16 in small plans (up to 64^3 points), which
+// would leave most of the device without a thread and wait on the longer chain.
+// Five C6 fields in us, 16 / 32: 160x129x96 y lines 60 / 40, 1000x300 x6 x lines
+// 22.5 / 12.8, 64^3 walls FP32 6.7 / 8.5.
+constexpr int64_t kLineWide = ((int64_t)1 << 18) + 1;
 
 void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
     const CompactParams& P = plan.P;
@@ -488,7 +490,7 @@ void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
                     if (periodic && R.nseg == S) a = ((a % S) + S) % S;
                     if (a < 0 || a >= R.nseg) continue;
                     for (int u = 0; u < b2; ++u)
-                        tab[(((size_t)s * b2 + side * q + t) * Wn + j) * b2 + u] =
+                        tab[line_row_index(MS, S, b2 * Wn * b2, ((side * q + t) * Wn + j) * b2 + u, s)] =
                             R.g[(size_t)r * b2 * R.nseg + b2 * a + u];
                 }
             }

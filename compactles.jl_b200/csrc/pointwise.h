@@ -68,6 +68,13 @@ struct BcState {
     int ew_times_T;   // ideal-mixture form of the wall energy
 };
 
+// The enforced faces of one apply_bcs! (cell-local conditions), in order.
+struct BcFaces {
+    int n;
+    int d[6], side[6], kind[6];
+    BcState st[6];
+};
+
 // One characteristic (NSCBC) face, parameters resolved on the host.
 struct NscbcParams {
     int kind;         // CLES_BC_NSCBC_OUTFLOW or CLES_BC_NSCBC_INFLOW
@@ -248,6 +255,8 @@ void rate_final(const double* part, int nb, double* out, cudaStream_t st);
 // qface: per-node conserved state ([c][plane]) of a DirichletBC(fun) face, else null
 void bc_plane(double* Q, const Grid3& g, int d, int side, int Ns, int kind, const BcState& s, cudaStream_t st,
               const double* qface = nullptr);
+// All of F's faces in one launch
+void bc_faces(double* Q, const Grid3& g, int Ns, const BcFaces& F, cudaStream_t st);
 // Interior of one padded field (extents n + 2 pad, x fastest) into the interior layout.
 void gather_interior(const double* padded, double* interior, const int n[3], const int pad[3], cudaStream_t st);
 

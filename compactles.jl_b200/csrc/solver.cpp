@@ -767,7 +767,10 @@ public:
     }
 
     void apply_bcs() override {
-        // apply_bcs! (src/boundary.jl:280-286): active dims, low then high face
+        // apply_bcs! (src/boundary.jl:280-286): active dims, low then high face.
+        // Conditions of one cell go in one launch; a face that reads its neighbour
+        // plane or a host function's values gets its own, in order.
+        BcFaces faces{};
         for (int k = 0; k < 3; ++k) {
             if (!g_.active[k]) continue;
             for (int s = 0; s < 2; ++s) {
@@ -788,11 +791,20 @@ public:
                         for (int sp = 0; sp < Ns_; ++sp)
                             bs.ew[sp] = desc.eos == CLES_EOS_IDEAL ? pc_.cvk[sp] : nasa9_species_energy(desc, sp, Tw);
                 }
-                const double* qface = nullptr;
-                if (bc == CLES_BC_DIRICHLET && face_fn(k, s).fn) qface = eval_face_fn(k, s, ncons_);
-                bc_plane(Q_.as<double>(), g_, k, s, Ns_, bc, bs, st_, qface);
+                const bool fn = bc == CLES_BC_DIRICHLET && face_fn(k, s).fn;
+                if (fn || bc == CLES_BC_EXTRAPOLATION) {
+                    bc_faces(Q_.as<double>(), g_, Ns_, faces, st_);
+                    faces.n = 0;
+                    bc_plane(Q_.as<double>(), g_, k, s, Ns_, bc, bs, st_, fn ? eval_face_fn(k, s, ncons_) : nullptr);
+                    continue;
+                }
+                faces.d[faces.n] = k;
+                faces.side[faces.n] = s;
+                faces.kind[faces.n] = bc;
+                faces.st[faces.n++] = bs;
             }
         }
+        bc_faces(Q_.as<double>(), g_, Ns_, faces, st_);
     }
 
     // correct_rhs! of the characteristic faces (src/rhs.jl:688-691), after the
@@ -881,12 +893,15 @@ public:
         // the boundary correction and the sources come between the divergence and the update
         if (nscbc || sources) rk = nullptr;
         if (!primitives_current) PW::primitives(Q_.as<double>(), prim_.as<F>(), cells_, Ns_, pc_, st_, desc.art_enabled);
-        velocity_gradients();
-        compute_artificial();
         // temperature and mass-fraction gradients (src/rhs.jl:628-636); with one
-        // species only dT (the species diffusion flux vanishes, see k_fluxes)
+        // species only dT (the species diffusion flux vanishes, see k_fluxes).  On
+        // small grids they share the velocity gradients' launches; on large ones they
+        // come right before the flux pass, which then finds them in L2.
         const int ngty = Ns_ == 1 ? 1 : 1 + Ns_;
-        for (int k = 0; k < 3; ++k)
+        const bool paired = cells_ <= ((int64_t)1 << 21) && !folded_ && !decomposed_;
+        velocity_gradients(paired ? ngty : 0);
+        compute_artificial();
+        for (int k = 0; k < 3 && !paired; ++k)
             if (g_.active[k])
                 along_set(dset_[k], k, prim(P_T), gty_.as<F>() + (size_t)cells_ * ngty * k, ngty, OUT_STORE, nullptr);
         if (geo_) {
@@ -979,12 +994,18 @@ public:
 
     // velocity gradients grad_u[d][j] (src/rhs.jl:596-604): one launch per dim
     // for u, v, w (per parity on a fold), then on curvilinear / stretched grids
-    // the 1/h_d scaling and the curvature terms
-    void velocity_gradients() {
-        for (int k = 0; k < 3; ++k)
-            if (g_.active[k])
-                along_set(dset_[k], k, prim(P_U), g_u_.as<F>() + (size_t)cells_ * 3 * k, 3, OUT_STORE,
-                          fold_[k].on ? fold_[k].sigvel : nullptr);
+    // the 1/h_d scaling and the curvature terms.  ngty > 0: the first ngty of T and
+    // Y_k in the same launches (not on folds or split dims).
+    void velocity_gradients(int ngty = 0) {
+        for (int k = 0; k < 3; ++k) {
+            if (!g_.active[k]) continue;
+            F* g = g_u_.as<F>() + (size_t)cells_ * 3 * k;
+            if (ngty > 0)
+                launch_compact_pair(*dset_[k][0], view(prim(P_U)), view(g), 3, view(prim(P_T)),
+                                    view(gty_.as<F>() + (size_t)cells_ * ngty * k), ngty, st_);
+            else
+                along_set(dset_[k], k, prim(P_U), g, 3, OUT_STORE, fold_[k].on ? fold_[k].sigvel : nullptr);
+        }
         if (geo_) MetricOps<F>::metric_grad(g_u_.as<F>(), prim_.as<F>(), G_, g_, st_);
     }
 
