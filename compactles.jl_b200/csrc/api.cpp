@@ -46,6 +46,13 @@ int prof_begin(cudaStream_t st, int family, double bytes) {
 }
 void prof_end(int rec, cudaStream_t st) { CLES_CUDA(cudaEventRecord(g_prof[rec].b, st)); }
 
+namespace {
+thread_local bool g_dependent = false;
+}
+DependentLaunches::DependentLaunches(bool on) : prev_(g_dependent) { g_dependent = on; }
+DependentLaunches::~DependentLaunches() { g_dependent = prev_; }
+bool DependentLaunches::active() { return g_dependent; }
+
 void set_last_error(const std::string& s) { g_last_error = s; }
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 int64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }

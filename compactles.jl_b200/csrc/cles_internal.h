@@ -7,6 +7,7 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/cles.h"
@@ -32,6 +33,49 @@ bool profiling();
 int prof_begin(cudaStream_t st, int family, double bytes);
 void prof_end(int rec, cudaStream_t st);
 void check_launch(const char* what);
+
+// -------------------------------------------------- dependent launches ----
+// Kernels of a step follow one another on one stream, a few microseconds each on
+// small grids.  Inside a DependentLaunches scope (one thread's launches, one
+// solver's step) they are launched with programmatic stream serialization: a
+// kernel's blocks may start while its predecessor drains, set up what does not
+// depend on it (indices, constant tables) and wait in grid_dependency_wait until
+// it has completed.  Only kernels that call it are launched so.
+struct DependentLaunches {
+    explicit DependentLaunches(bool on);
+    ~DependentLaunches();
+    DependentLaunches(const DependentLaunches&) = delete;
+    static bool active();
+
+private:
+    bool prev_;
+};
+#ifdef __CUDACC__
+// Until every earlier kernel of the stream has completed (at once when launched
+// normally); lets the next kernel's blocks come in behind this one's.
+__device__ __forceinline__ void grid_dependency_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Launch of a kernel that calls grid_dependency_wait before it touches anything
+// another kernel writes.
+template <typename... K, typename... A>
+inline void launch_dependent(void (*kern)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (DependentLaunches::active()) {
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+    }
+    CLES_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
+}
+#endif
 
 // ------------------------------------------------------------ field views ----
 // A batch of scalar fields of one grid: element (i, j, k) of field b sits at

@@ -69,6 +69,7 @@ __device__ __forceinline__ T wl(const double* d, const float* f, int i) {
 template <typename T, int M, int XP>
 __global__ void __launch_bounds__(256) k_compact_xw(const __grid_constant__ CompactParams P, const __grid_constant__ WarpLineParams W, const FieldView in,
                                                     const FieldView out, const int mode) {
+    grid_dependency_wait();
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int line = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -172,17 +173,18 @@ void launch_xw_m(const CompactPlan& plan, const FieldView& in, const FieldView& 
                  cudaStream_t st) {
     const int lines_per_cta = 8;
     dim3 grid((unsigned)((plan.P.lines + lines_per_cta - 1) / lines_per_cta), (unsigned)count);
+    auto go = [&](auto kern) { launch_dependent(kern, grid, dim3(32 * lines_per_cta), 0, st, plan.P, plan.XW, in, out, mode); };
     switch (plan.XW.XP) {
         case 2:
             // the stencil halo comes from the neighbouring lanes' XP points: XP >= M
-            if constexpr (M <= 2) k_compact_xw<T, M, 2><<<grid, 32 * lines_per_cta, 0, st>>>(plan.P, plan.XW, in, out, mode);
+            if constexpr (M <= 2) go(k_compact_xw<T, M, 2>);
             else throw Error(CLES_EINVAL, "warp-line kernel: fewer points per lane than the stencil half-width");
             break;
-        case 4: k_compact_xw<T, M, 4><<<grid, 32 * lines_per_cta, 0, st>>>(plan.P, plan.XW, in, out, mode); break;
-        case 6: k_compact_xw<T, M, 6><<<grid, 32 * lines_per_cta, 0, st>>>(plan.P, plan.XW, in, out, mode); break;
-        case 8: k_compact_xw<T, M, 8><<<grid, 32 * lines_per_cta, 0, st>>>(plan.P, plan.XW, in, out, mode); break;
-        case 12: k_compact_xw<T, M, 12><<<grid, 32 * lines_per_cta, 0, st>>>(plan.P, plan.XW, in, out, mode); break;
-        case 16: k_compact_xw<T, M, 16><<<grid, 32 * lines_per_cta, 0, st>>>(plan.P, plan.XW, in, out, mode); break;
+        case 4: go(k_compact_xw<T, M, 4>); break;
+        case 6: go(k_compact_xw<T, M, 6>); break;
+        case 8: go(k_compact_xw<T, M, 8>); break;
+        case 12: go(k_compact_xw<T, M, 12>); break;
+        case 16: go(k_compact_xw<T, M, 16>); break;
         default: throw Error(CLES_EINVAL, "warp-line kernel: unsupported points per lane");
     }
     count_launch();
@@ -291,14 +293,16 @@ bool try_launch_line(const CompactPlan& plan, const FieldView& in, const FieldVi
 
 // Which kernel a line solve takes.  Periodic tridiagonal x lines of 32 k points:
 // a warp per line.  y / z lines whose equal segments fill a TMA tile: the
-// tile kernels, from 128 points (periodic tridiagonal) and 160 points (closed, or
-// C10) on: shorter lines leave a tile CTA with four warps or fewer.  Everything
-// else: k_line.  Schemes whose interface system decays too slowly for its window
+// tile kernels from 160 points on (shorter lines leave a tile CTA with four warps
+// or fewer: three periodic C6 fields of 128^3 25.4 us against 22.6 for k_line; FP64
+// closed lines of 192 points 74 against 87 us), FP32 closed and C10 lines from 224
+// (192 points: 92 against 87 us for five filtered fields; 256: 132 against 156).
+// Everything else: k_line.  Schemes whose interface system decays too slowly for its window
 // have no k_line form and take the tile kernels where they fit, else the generic
 // one.
 static bool tile_first(const CompactPlan& plan) {
     const CompactParams& P = plan.P;
-    return P.dim > 0 && P.n >= (plan.has_tl ? 128 : 160);
+    return P.dim > 0 && P.n >= (plan.has_tl || plan.dtype == CLES_F64 ? 160 : 224);
 }
 
 void launch_compact(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,

@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(MS == 16 ? 512 : 256, CPS)
     }
     for (int i = tid; i < N * N; i += blockDim.x) Gs[i] = Gg[i];
     __syncthreads();
+    grid_dependency_wait();
 
     const unsigned tile_bytes = (unsigned)(sizeof(T) * tile_elems);
     auto issue = [&](int w, int s) {
@@ -447,6 +448,7 @@ __global__ void __launch_bounds__(256, 2)
     }
     for (int i = tid; i < N * N; i += blockDim.x) Gs[i] = tab[P.off_G + i];
     __syncthreads();
+    grid_dependency_wait();
 
     const unsigned tile_bytes = (unsigned)(sizeof(T) * tile_elems);
     auto issue = [&](int w, int s) {
@@ -891,7 +893,7 @@ void launch_tma_ms(const CompactPlan& plan, const CUtensorMap& map, const FieldV
     const int work = gx * (P.dim == 1 ? P.nz : P.ny) * count;
     const int slots = g_num_sms * (2 * (smem + 1024) <= 227 * 1024 ? per_sm : 1);
     const int grid = work < slots ? work : slots;
-    kern<<<grid, kLanes * P.S, smem, st>>>(map, P, plan.TL, G, out, mode, count, NS, rk);
+    launch_dependent(kern, dim3(grid), dim3(kLanes * P.S), smem, st, map, P, plan.TL, G, out, mode, count, NS, rk);
     count_launch();
     check_launch("k_compact_tma");
 }
@@ -945,7 +947,8 @@ void launch_tg_ms(const CompactPlan& plan, const CUtensorMap& map, const FieldVi
     if (per_sm < 1) per_sm = 1;
     const int slots = g_num_sms * per_sm;
     const int grid = work < slots ? work : slots;
-    kern<<<grid, kLanes * P.S, smem, st>>>(map, P, plan.TG, tab, out, mode, count, NS, rk, H, iface);
+    launch_dependent(kern, dim3(grid), dim3(kLanes * P.S), smem, st, map, P, plan.TG, tab, out, mode, count, NS, rk, H,
+                     iface);
     count_launch();
     check_launch("k_compact_tg");
 }

@@ -41,6 +41,7 @@ __device__ __forceinline__ double jl_min(double x, double y) {
 // g[3 d + j] = d u_j / d x_d.
 template <typename F>
 __global__ void k_metric_grad(F* __restrict__ g, const F* __restrict__ prim, Geom G, Grid3 gr, int64_t cells) {
+    grid_dependency_wait();
     GRID_STRIDE(I, cells) {
         int i, j, k;
         cell_ijk(I, gr.n, i, j, k);
@@ -73,6 +74,7 @@ __global__ void k_metric_grad(F* __restrict__ g, const F* __restrict__ prim, Geo
 // _scale_grad! (src/rhs.jl:477-483) of `count` fields per active dim
 template <typename F>
 __global__ void k_scale_grad(F* __restrict__ f, int count, Geom G, Grid3 gr, int64_t cells) {
+    grid_dependency_wait();
     GRID_STRIDE(I, cells) {
         int i, j, k;
         cell_ijk(I, gr.n, i, j, k);
@@ -108,6 +110,7 @@ template <typename F>
 __global__ void k_metric_div(F* __restrict__ dQ, const F* __restrict__ fd, int ncons, int Ns,
                              const F* __restrict__ prim, const F* __restrict__ g, const F* __restrict__ art,
                              double mu0, Geom G, Grid3 gr, int64_t cells) {
+    grid_dependency_wait();
     GRID_STRIDE(I, cells) {
         int i, j, k;
         cell_ijk(I, gr.n, i, j, k);
@@ -272,14 +275,14 @@ __global__ void k_geo_gcl(double* __restrict__ cotr, const double* __restrict__ 
 template <typename F>
 void MetricOps<F>::metric_grad(F* g, const F* prim, const Geom& G, const Grid3& gr, cudaStream_t st) {
     const int64_t cells = (int64_t)gr.n[0] * gr.n[1] * gr.n[2];
-    k_metric_grad<F><<<grid_for(cells), kThreads, 0, st>>>(g, prim, G, gr, cells);
+    launch_dependent(k_metric_grad<F>, dim3(grid_for(cells)), dim3(kThreads), 0, st, g, prim, G, gr, cells);
     count_launch();
     check_launch("k_metric_grad");
 }
 template <typename F>
 void MetricOps<F>::scale_grad(F* f, int count, const Geom& G, const Grid3& gr, cudaStream_t st) {
     const int64_t cells = (int64_t)gr.n[0] * gr.n[1] * gr.n[2];
-    k_scale_grad<F><<<grid_for(cells), kThreads, 0, st>>>(f, count, G, gr, cells);
+    launch_dependent(k_scale_grad<F>, dim3(grid_for(cells)), dim3(kThreads), 0, st, f, count, G, gr, cells);
     count_launch();
     check_launch("k_scale_grad");
 }
@@ -287,7 +290,7 @@ template <typename F>
 void MetricOps<F>::metric_div(F* dQ, const F* fd, int ncons, int Ns, const F* prim, const F* g, const F* art,
                               double mu0, const Geom& G, const Grid3& gr, cudaStream_t st) {
     const int64_t cells = (int64_t)gr.n[0] * gr.n[1] * gr.n[2];
-    k_metric_div<F><<<grid_for(cells), kThreads, 0, st>>>(dQ, fd, ncons, Ns, prim, g, art, mu0, G, gr, cells);
+    launch_dependent(k_metric_div<F>, dim3(grid_for(cells)), dim3(kThreads), 0, st, dQ, fd, ncons, Ns, prim, g, art, mu0, G, gr, cells);
     count_launch();
     check_launch("k_metric_div");
 }

@@ -238,6 +238,7 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
         ln_stage(csm, reinterpret_cast<const T*>(C), (int)(sizeof(Coef) / sizeof(T)));
         if (A.gstage) ln_stage(gsm, Gw, 2 * Q * A.Wn * 2 * Q * S);
     }
+    grid_dependency_wait();   // the tables above are constant
 
     // element offset of point 0 of x line l
     auto line_base = [&](const FieldView& v, int l) -> int64_t {
@@ -720,14 +721,18 @@ void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView
     cfg.blockDim = dim3((unsigned)((s.L * s.SC + 31) / 32 * 32));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
+    cfg.attrs = at;
     if (s.CL > 1) {
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = (unsigned)s.CL;
         at[0].val.clusterDim.y = 1;
         at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
         cfg.numAttrs = 1;
+    }
+    if (DependentLaunches::active()) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
     const void* tab = lp.tab;
     const void* dcoef = lp.dcoef;

@@ -93,6 +93,14 @@ inline unsigned grid_for(int64_t n) {
         check_launch(#kern);                                           \
     } while (0)
 
+// the same for a kernel that starts with grid_dependency_wait
+#define LAUNCH_DEP(kern, n, st, ...)                                                   \
+    do {                                                                                \
+        launch_dependent(kern, dim3(grid_for(n)), dim3(kThreads), 0, st, __VA_ARGS__);  \
+        count_launch();                                                                 \
+        check_launch(#kern);                                                            \
+    } while (0)
+
 #define GRID_STRIDE(idx, n) for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < (n); idx += (int64_t)gridDim.x * blockDim.x)
 
 // Constants of the max_rate reduction (src/timestep.jl:125-175), Cartesian.
@@ -160,6 +168,7 @@ __global__ void __launch_bounds__(kThreads, RATE ? 3 : 4) k_primitives(const dou
                              int esens, const double* __restrict__ mc = nullptr, const int* __restrict__ tmap = nullptr,
                              const F* __restrict__ art = nullptr, double* __restrict__ part = nullptr,
                              const RateConst rc = RateConst{}) {
+    grid_dependency_wait();
     double rate = 0.0, rmin = __longlong_as_double(0x7ff0000000000000LL);
     GRID_STRIDE(I, cells) {
         const double* mcI = nullptr;
@@ -244,6 +253,7 @@ __global__ void __launch_bounds__(kThreads, RATE ? 3 : 4) k_primitives(const dou
 // on 256^3 FP64 cells 766 -> 1572 us).
 template <typename F, int DIMS>
 __global__ void k_strain(const F* __restrict__ g, F* __restrict__ out, int64_t cells) {
+    grid_dependency_wait();
     GRID_STRIDE(I, cells) {
         double gv[9];
 #pragma unroll
@@ -403,6 +413,7 @@ __device__ __forceinline__ void delta4_tile(const F* __restrict__ f0, F* __restr
 
 template <typename F>
 __global__ void __launch_bounds__(kD4Threads) k_delta4(const D4Set<F> fs, Grid3 g, Weights3 h, int nzc, int nchunks) {
+    grid_dependency_wait();
     const int f = blockIdx.z / nchunks, zc = blockIdx.z - f * nchunks;
     Weights3 w;
     for (int d = 0; d < 3; ++d) w.w[d] = fs.p[f] == 2 ? h.w[d] * h.w[d] : h.w[d];
@@ -478,6 +489,7 @@ template <typename F>
 __global__ void k_art_coef(const F* __restrict__ sens, const F* __restrict__ prim, const F* __restrict__ g,
                            F* __restrict__ art, int64_t cells, int Ns, double C_mu, double C_beta, double C_kappa,
                            double C_D, int gate) {
+    grid_dependency_wait();
     GRID_STRIDE(I, cells) {
         const double rho = double(prim[I + cells * P_RHO]);
         const double c = double(prim[I + cells * P_C]);
@@ -532,6 +544,7 @@ __global__ void k_fluxes(const double* __restrict__ Q, const F* __restrict__ pri
                          const F* __restrict__ gty, const F* __restrict__ art, F* __restrict__ flux, int64_t cells,
                          int Ns, PhysConst pc, double mu0, double Pr, double Sc, Geom G,
                          const double* __restrict__ mc = nullptr, const int* __restrict__ tmap = nullptr) {
+    grid_dependency_wait();
     if (SINGLE) Ns = 1;
     const int ncons = Ns + 4;
     const int gstride = SINGLE ? 1 : 1 + Ns;
@@ -635,6 +648,7 @@ __global__ void k_body_forces(F* __restrict__ dQ, const double* __restrict__ Q, 
 template <typename F>
 __global__ void k_lsrk(double* __restrict__ Q, double* __restrict__ du, const F* __restrict__ dQ, int64_t n, double A,
                        double B, double dt, const double* __restrict__ dtp) {
+    grid_dependency_wait();
     if (dtp) dt = *dtp;
     GRID_STRIDE(I, n) {
         const double v = A * du[I] + dt * double(dQ[I]);
@@ -644,6 +658,7 @@ __global__ void k_lsrk(double* __restrict__ Q, double* __restrict__ du, const F*
 }
 
 __global__ void k_rate_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
+    grid_dependency_wait();
     __shared__ double sr[kThreads], sm[kThreads];
     double rate = 0.0, rmin = __longlong_as_double(0x7ff0000000000000LL);
     for (int b = threadIdx.x; b < nb; b += blockDim.x) {
@@ -818,6 +833,7 @@ __global__ void k_bc_plane(double* __restrict__ Q, Grid3 g, int d, int side, int
 // ascending, low face first).  Six faces of a 129^3 box: 6 x 5 us as launches of
 // their own.
 __global__ void k_bc_faces(double* __restrict__ Q, Grid3 g, int Ns, const __grid_constant__ BcFaces F) {
+    grid_dependency_wait();
     const int f = blockIdx.y, d = F.d[f];
     const int64_t cells = (int64_t)g.n[0] * g.n[1] * g.n[2];
     const int o1 = d == 0 ? 1 : 0, o2 = d == 2 ? 1 : 2;
@@ -985,6 +1001,7 @@ __device__ __forceinline__ void clock_before_body(double* __restrict__ clk, cons
     clk[DC_DT] = jl_min(dt, c.tfinal - clk[DC_T]);
 }
 __global__ void k_clock_before(double* __restrict__ clk, const double* __restrict__ rate_rmin, ClockConst c) {
+    grid_dependency_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     clock_before_body(clk, rate_rmin[0], rate_rmin[1], c);
 }
@@ -996,6 +1013,7 @@ __device__ __forceinline__ void clock_after_body(double* __restrict__ clk, const
     if (!(clk[DC_T] < c.tfinal) || !(clk[DC_STEP] < c.nmax)) clk[DC_DONE] = 1.0;
 }
 __global__ void k_clock_after(double* __restrict__ clk, ClockConst c) {
+    grid_dependency_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     clock_after_body(clk, c);
 }
@@ -1087,7 +1105,7 @@ __global__ void k_clock_after_batch(const BatchGrid* __restrict__ grids, int G) 
 }  // namespace
 
 void clock_before(double* clk, const double* rate_rmin, const ClockConst& c, cudaStream_t st) {
-    k_clock_before<<<1, 32, 0, st>>>(clk, rate_rmin, c);
+    launch_dependent(k_clock_before, dim3(1), dim3(32), 0, st, clk, rate_rmin, c);
     count_launch();
     check_launch("k_clock_before");
 }
@@ -1113,16 +1131,16 @@ void BatchOps<F>::rate_clock(const double* Q, const F* prim, const F* art, const
 template <typename F>
 void BatchOps<F>::primitives(const double* Q, F* prim, int64_t ct, int Ns, const PhysConst& pc, int esens,
                              const double* mc, const int* tmap, cudaStream_t st) {
-    LAUNCH((k_primitives<F, false, true>), ct, st, Q, prim, ct, Ns, pc, esens, mc, tmap, nullptr, nullptr, RateConst{});
+    LAUNCH_DEP((k_primitives<F, false, true>), ct, st, Q, prim, ct, Ns, pc, esens, mc, tmap, nullptr, nullptr, RateConst{});
 }
 // k_fluxes for the active dimensions: 1-D and 2-D grids along x and y have their
 // own instantiations, any other set runs all three directions (the gradients of a
 // collapsed dimension are zero, its flux is not read)
 #define LAUNCH_FLUXES(F, SINGLE, N9, GEO, PM, n, st, ...)                                \
     do {                                                                                 \
-        if (dims == 1) LAUNCH((k_fluxes<F, SINGLE, N9, GEO, PM, 1>), n, st, __VA_ARGS__); \
-        else if (dims == 3) LAUNCH((k_fluxes<F, SINGLE, N9, GEO, PM, 3>), n, st, __VA_ARGS__); \
-        else LAUNCH((k_fluxes<F, SINGLE, N9, GEO, PM, 7>), n, st, __VA_ARGS__);           \
+        if (dims == 1) LAUNCH_DEP((k_fluxes<F, SINGLE, N9, GEO, PM, 1>), n, st, __VA_ARGS__); \
+        else if (dims == 3) LAUNCH_DEP((k_fluxes<F, SINGLE, N9, GEO, PM, 3>), n, st, __VA_ARGS__); \
+        else LAUNCH_DEP((k_fluxes<F, SINGLE, N9, GEO, PM, 7>), n, st, __VA_ARGS__);           \
     } while (0)
 template <typename F>
 void BatchOps<F>::fluxes(const double* Q, const F* prim, const F* g, const F* gty, const F* art, F* flux, int64_t ct,
@@ -1158,7 +1176,7 @@ void batch_clock_after(const BatchGrid* grids, int G, cudaStream_t st) {
 }
 
 void clock_after(double* clk, const ClockConst& c, cudaStream_t st) {
-    k_clock_after<<<1, 32, 0, st>>>(clk, c);
+    launch_dependent(k_clock_after, dim3(1), dim3(32), 0, st, clk, c);
     count_launch();
     check_launch("k_clock_after");
 }
@@ -1168,8 +1186,8 @@ void clock_after(double* clk, const ClockConst& c, cudaStream_t st) {
 template <typename F>
 void Pointwise<F>::primitives(const double* Q, F* prim, int64_t cells, int Ns, const PhysConst& pc, cudaStream_t st,
                               int esens) {
-    if (pc.eos == CLES_EOS_NASA9) LAUNCH((k_primitives<F, true>), cells, st, Q, prim, cells, Ns, pc, esens, nullptr, nullptr, nullptr, nullptr, RateConst{});
-    else LAUNCH((k_primitives<F, false>), cells, st, Q, prim, cells, Ns, pc, esens, nullptr, nullptr, nullptr, nullptr, RateConst{});
+    if (pc.eos == CLES_EOS_NASA9) LAUNCH_DEP((k_primitives<F, true>), cells, st, Q, prim, cells, Ns, pc, esens, nullptr, nullptr, nullptr, nullptr, RateConst{});
+    else LAUNCH_DEP((k_primitives<F, false>), cells, st, Q, prim, cells, Ns, pc, esens, nullptr, nullptr, nullptr, nullptr, RateConst{});
 }
 // Planes a block walks: 32 (the four planes of run-in cost an eighth), fewer
 // where the launch would leave the SMs with less than four blocks of 256 threads
@@ -1182,7 +1200,7 @@ void Pointwise<F>::delta4(const D4Set<F>& fs, const Grid3& g, const double h[3],
     while (nzc > 8 && (int64_t)bx * by * ((g.n[2] + nzc - 1) / nzc) * fs.n < 4 * num_sms()) nzc /= 2;
     const int nchunks = (g.n[2] + nzc - 1) / nzc;
     const dim3 grid((unsigned)bx, (unsigned)by, (unsigned)(nchunks * fs.n));
-    k_delta4<F><<<grid, kD4Threads, 0, st>>>(fs, g, Weights3{{h[0], h[1], h[2]}}, nzc, nchunks);
+    launch_dependent(k_delta4<F>, grid, dim3(kD4Threads), 0, st, fs, g, Weights3{{h[0], h[1], h[2]}}, nzc, nchunks);
     count_launch();
     check_launch("k_delta4");
 }
@@ -1201,14 +1219,14 @@ void Pointwise<F>::delta4_halo(const F* f0, const F* f1, F* o0, F* o1, const Gri
 template <typename F>
 void Pointwise<F>::art_coef(const F* sens, const F* prim, const F* g, F* art, int64_t cells, int Ns, double C_mu,
                             double C_beta, double C_kappa, double C_D, int gate, cudaStream_t st) {
-    LAUNCH(k_art_coef<F>, cells, st, sens, prim, g, art, cells, Ns, C_mu, C_beta, C_kappa, C_D, gate);
+    LAUNCH_DEP(k_art_coef<F>, cells, st, sens, prim, g, art, cells, Ns, C_mu, C_beta, C_kappa, C_D, gate);
 }
 template <typename F>
 void Pointwise<F>::strain(const F* g, F* out, int64_t cells, int dims, cudaStream_t st) {
     switch (dims) {
-        case 1: LAUNCH((k_strain<F, 1>), cells, st, g, out, cells); break;
-        case 3: LAUNCH((k_strain<F, 3>), cells, st, g, out, cells); break;
-        default: LAUNCH((k_strain<F, 7>), cells, st, g, out, cells);
+        case 1: LAUNCH_DEP((k_strain<F, 1>), cells, st, g, out, cells); break;
+        case 3: LAUNCH_DEP((k_strain<F, 3>), cells, st, g, out, cells); break;
+        default: LAUNCH_DEP((k_strain<F, 7>), cells, st, g, out, cells);
     }
 }
 template <typename F>
@@ -1256,7 +1274,7 @@ void Pointwise<F>::body_forces(F* dQ, const double* Q, int64_t cells, int Ns, co
 template <typename F>
 void Pointwise<F>::lsrk(double* Q, double* du, const F* dQ, int64_t n, double A, double B, double dt, cudaStream_t st,
                         const double* dtp) {
-    LAUNCH(k_lsrk<F>, n, st, Q, du, dQ, n, A, B, dt, dtp);
+    LAUNCH_DEP(k_lsrk<F>, n, st, Q, du, dQ, n, A, B, dt, dtp);
 }
 template <typename F>
 void Pointwise<F>::primitives_rate(const double* Q, F* prim, const F* art, double* part, double* out, int64_t cells,
@@ -1265,17 +1283,17 @@ void Pointwise<F>::primitives_rate(const double* Q, F* prim, const F* art, doubl
     const RateConst R{{idx[0], idx[1], idx[2]}, {act[0], act[1], act[2]}, mu0, mu0 / Pr, mu0 / Sc};
     const unsigned nb = (unsigned)rate_partials(cells);
     if (pc.eos == CLES_EOS_NASA9)
-        k_primitives<F, true, false, true><<<nb, kThreads, 0, st>>>(Q, prim, cells, Ns, pc, esens, nullptr, nullptr, art,
-                                                                    part, R);
+        launch_dependent(k_primitives<F, true, false, true>, dim3(nb), dim3(kThreads), 0, st, Q, prim, cells, Ns, pc,
+                         esens, nullptr, nullptr, art, part, R);
     else
-        k_primitives<F, false, false, true><<<nb, kThreads, 0, st>>>(Q, prim, cells, Ns, pc, esens, nullptr, nullptr,
-                                                                     art, part, R);
+        launch_dependent(k_primitives<F, false, false, true>, dim3(nb), dim3(kThreads), 0, st, Q, prim, cells, Ns, pc,
+                         esens, nullptr, nullptr, art, part, R);
     count_launch();
     check_launch("k_primitives");
     rate_final(part, (int)nb, out, st);
 }
 void rate_final(const double* part, int nb, double* out, cudaStream_t st) {
-    k_rate_final<<<1, kThreads, 0, st>>>(part, nb, out);
+    launch_dependent(k_rate_final, dim3(1), dim3(kThreads), 0, st, part, nb, out);
     count_launch();
     check_launch("k_rate_final");
 }
@@ -1315,7 +1333,7 @@ void bc_faces(double* Q, const Grid3& g, int Ns, const BcFaces& F, cudaStream_t 
             if (e != F.d[f]) p *= g.n[e];
         most = std::max(most, p);
     }
-    k_bc_faces<<<dim3(grid_for(most), (unsigned)F.n), kThreads, 0, st>>>(Q, g, Ns, F);
+    launch_dependent(k_bc_faces, dim3(grid_for(most), (unsigned)F.n), dim3(kThreads), 0, st, Q, g, Ns, F);
     count_launch();
     check_launch("k_bc_faces");
 }
