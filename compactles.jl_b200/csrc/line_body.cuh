@@ -17,12 +17,24 @@
 // neither a wide block nor a second launch, and a store in place is safe since
 // every block has read its points before the cluster barrier.
 //
+// What bounds it: large plans in FP64 the registers (128 a thread, 16 warps an SM:
+// load, solve and store phases of the resident blocks cover each other only in
+// part), in FP32 instruction issue; small plans latency.  Against the kernels it
+// replaced (generic segments with table loads; two launches of pieces for few long
+// lines), us a launch on B200:
+//   C10, three FP64 201x161x129 fields, walls, x / y / z: 243 / 166 / 136 -> 98 / 80 / 72
+//   C6, five FP64 129^3 fields, walls: 154 / 86 / 86 -> 64 / 48 / 49
+//   C6, six FP64 2048x1024 fields, walls, x / y: 211 / 120 -> 69 / 69
+//   C8 filter, five FP32 256x192x160 fields, walls, x: 130 -> 99
+//   C6, six FP64 lines of 5712 points: 18.9 -> 10.7
+//
 // XM = false (y, z lines): lanes are consecutive x, the window is read straight
 // from global memory.  XM = true (x lines): the block's rows are staged by
 // cp.async into shared rows of odd pitch, so that both the row-wise copies and
 // the threads' walks along their segments are free of bank conflicts.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "cles_internal.h"
@@ -643,8 +655,11 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
 // contiguous, and 16 FP64 y / z lanes still fill 128-byte rows; FP32 y / z lines
 // keep 32), else the line over a cluster of up to 8 blocks.  Fewer lines a block
 // where the launch would not fill the SMs twice: down to 8 (64-byte rows) along y
-// and z, 1 along x; and one block of up to 512 threads rather than a cluster where
-// it cannot fill them once.
+// and z, 1 along x.  Where it cannot fill them once, a block that would have more
+// than 256 threads is cut into a cluster of 64-thread ones, whose SMs load and
+// solve side by side: 20 steps of a 5712-cell tube 5.84 ms as one block a line,
+// 5.73 as blocks of 256, 5.40 of 128, 4.90 of 64; lines of 1000 cells gain nothing
+// (8.6 us a launch, 9.6 cut).
 struct LineShape {
     int L, SC, CL;
 };
@@ -666,7 +681,12 @@ inline LineShape line_shape(const CompactParams& P, const LinePlan& lp, int coun
     auto blocks = [&](int l) { return ((P.lines + l - 1) / l) * count * shape(l).CL; };
     while (L > lmin && blocks(L) < 2 * num_sms) L /= 2;
     LineShape s = shape(L);
-    if (s.CL > 1 && lp.S * L <= 512 && blocks(L) < num_sms) s = LineShape{L, lp.S, 1};
+    if (blocks(L) < num_sms) {
+        const int threads = lp.S * L > 256 ? 64 : 256;
+        s.CL = std::min(8, (lp.S * L + threads - 1) / threads);
+        s.SC = (lp.S + s.CL - 1) / s.CL;
+        s.CL = (lp.S + s.SC - 1) / s.SC;
+    }
     return s;
 }
 

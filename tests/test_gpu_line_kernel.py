@@ -98,7 +98,7 @@ def test_rhs_and_steps(orc, n, walls):
     tp = 2 * np.pi
 
     def ic(x, y, z):
-        s = np.sin(tp * x) * np.cos(tp * y) + 0 * z
+        s = 0.7 * np.sin(tp * x + 0.7) * np.cos(tp * y + 0.4) + 0.3 * np.sin(tp * z + 0.2)
         Y = 0.5 + 0.3 * s
         return cl.Prim(u=(0.3 * s, 0.2 * s if n[1] > 1 else 0 * s, 0.1 * s if n[2] > 1 else 0 * s), p=2 + 0.2 * s,
                        rho=1 + 0.1 * s, Y=(Y, 1 - Y))
@@ -116,3 +116,33 @@ def test_rhs_and_steps(orc, n, walls):
     assert O.run(1e9, 5)[0] == 0
     qa, qb = S.get_state()[sl], O.get_state()[sl]
     assert np.linalg.norm(qa - qb) < 1e-11 * np.linalg.norm(qb)
+
+
+@pytest.mark.parametrize("n", [(1, 61, 1), (41, 1, 38), (1, 44, 39)])
+def test_other_collapsed_dimensions(orc, n):
+    """Grids whose collapsed dimension is not the last: every direction's code path runs."""
+    test_rhs_and_steps(orc, n, True)
+
+
+def test_mixed_faces_share_edges(orc):
+    """Enforced faces of different kinds in one launch: cells on edges and corners
+    get every face's condition in apply_bcs! order; an extrapolation face in between
+    keeps its place.  Bitwise against one condition at a time would need the oracle's
+    own rounding, hence 1e-14 of the largest value."""
+    n = (20, 18, 17)
+    D = cl.DirichletBC(cl.Prim(u=(0.1, 0.2, -0.1), p=1.3, rho=0.9))
+    for bcs in (((cl.SlipWallBC(), cl.NoSlipWallBC()), (D, cl.SlipWallBC()), (cl.NoSlipWallBC(Twall=1.1), D)),
+                ((cl.NoSlipWallBC(), cl.SlipWallBC()), (cl.ExtrapolationBC(), D), (cl.SlipWallBC(), cl.NoSlipWallBC()))):
+        mk = lambda m: cl.solver_desc(n, (1.0, 1.0, 1.0), bcs, m.lele_d1_6(), m.compact_filter(0.45))
+        dg, do = mk(cl), mk(orc)
+        rng = np.random.default_rng(3)
+        Q0 = cl.initialize(dg, lambda x, y, z: cl.Prim(u=tuple(0.3 * rng.standard_normal(n[::-1]) for _ in range(3)),
+                                                       p=2 + 0.1 * rng.random(n[::-1]), rho=1 + 0.1 * rng.random(n[::-1])))
+        sl = (slice(None),) + cl.interior_slices(dg)
+        S, O = cl.Solver(dg), orc.Solver(do)
+        S.set_state(Q0)
+        O.set_state(Q0)
+        S.apply_bcs()
+        O.apply_bcs()
+        a, b = S.get_state()[sl], O.get_state()[sl]
+        assert np.abs(a - b).max() <= 1e-14 * np.abs(b).max()
