@@ -51,11 +51,10 @@ __device__ __forceinline__ void ln_cp_async(double* dst, const double* src) {
 __device__ __forceinline__ void ln_cp_async(float* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(ln_smem(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void ln_cluster_arrive() { asm volatile("barrier.cluster.arrive;" ::: "memory"); }
-__device__ __forceinline__ void ln_cluster_arrive_relaxed() {
-    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
-}
-__device__ __forceinline__ void ln_cluster_wait() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
+// release / acquire: both barriers of the kernel order shared-memory accesses
+// across blocks
+__device__ __forceinline__ void ln_cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void ln_cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 // shared-window address of `addr` in block `rank` of the cluster
 __device__ __forceinline__ unsigned ln_map(unsigned addr, unsigned rank) {
     unsigned r;
@@ -505,9 +504,10 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
             zn[t] = an[t];
         }
     }
-    // no block leaves while another may still read its end values (nothing to
-    // publish: a relaxed arrival)
-    if (CL > 1) ln_cluster_arrive_relaxed();
+    // No block leaves while another may still read its end values: the arrival
+    // releases this block's remote reads above, the wait at the end of the kernel
+    // acquires those of the others.  The correction and the stores come in between.
+    if (CL > 1) ln_cluster_arrive();
     if constexpr (CS) {
         ln_correct<T, Q, MS>(LnShared<T, Q, MS>((ln_coef<T, Q, MS>(C, csm)), cls), mm, y, zp, zn);
     } else {
