@@ -41,6 +41,10 @@ void check_launch(const char* what);
 // kernel's blocks may start while its predecessor drains, set up what does not
 // depend on it (indices, constant tables) and wait in grid_dependency_wait until
 // it has completed.  Only kernels that call it are launched so.
+// Such a kernel is alive while its predecessor still writes, so its pointer
+// parameters carry no __restrict__ (that promises memory nobody else writes for the
+// kernel's whole life, and lets reads move above the wait).  The promise is made
+// to an inlined body called after the wait; constant plan tables keep it.
 struct DependentLaunches {
     explicit DependentLaunches(bool on);
     ~DependentLaunches();

@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(256, 2)
     k_compact_tg(const __grid_constant__ CUtensorMap map, const __grid_constant__ CompactParams P,
                  const __grid_constant__ TileGenParams GP, const T* __restrict__ tab, const FieldView out,
                  const int mode, const int count, const int NS, const RkEpilogue rk, const int H,
-                 T* __restrict__ iface) {
+                 T* iface) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int n = P.n, S = P.S;
     constexpr int m = MS;  // points per segment (all segments equal at launch)

@@ -40,8 +40,8 @@ __device__ __forceinline__ double jl_min(double x, double y) {
 // additive curvature terms of metric_correct_gradients! (src/metric.jl:181-221).
 // g[3 d + j] = d u_j / d x_d.
 template <typename F>
-__global__ void k_metric_grad(F* __restrict__ g, const F* __restrict__ prim, Geom G, Grid3 gr, int64_t cells) {
-    grid_dependency_wait();
+__device__ __forceinline__ void metric_grad_body(F* __restrict__ g, const F* __restrict__ prim, const Geom& G,
+                                                 const Grid3& gr, int64_t cells) {
     GRID_STRIDE(I, cells) {
         int i, j, k;
         cell_ijk(I, gr.n, i, j, k);
@@ -70,11 +70,17 @@ __global__ void k_metric_grad(F* __restrict__ g, const F* __restrict__ prim, Geo
         for (int e = 0; e < 9; ++e) g[I + cells * e] = F(gv[e]);
     }
 }
+template <typename F>
+__global__ void k_metric_grad(F* g, const F* prim, const __grid_constant__ Geom G, const __grid_constant__ Grid3 gr,
+                              int64_t cells) {
+    grid_dependency_wait();
+    metric_grad_body<F>(g, prim, G, gr, cells);
+}
 
 // _scale_grad! (src/rhs.jl:477-483) of `count` fields per active dim
 template <typename F>
-__global__ void k_scale_grad(F* __restrict__ f, int count, Geom G, Grid3 gr, int64_t cells) {
-    grid_dependency_wait();
+__device__ __forceinline__ void scale_grad_body(F* __restrict__ f, int count, const Geom& G, const Grid3& gr,
+                                                int64_t cells) {
     GRID_STRIDE(I, cells) {
         int i, j, k;
         cell_ijk(I, gr.n, i, j, k);
@@ -87,6 +93,12 @@ __global__ void k_scale_grad(F* __restrict__ f, int count, Geom G, Grid3 gr, int
             }
         }
     }
+}
+template <typename F>
+__global__ void k_scale_grad(F* f, int count, const __grid_constant__ Geom G, const __grid_constant__ Grid3 gr,
+                             int64_t cells) {
+    grid_dependency_wait();
+    scale_grad_body<F>(f, count, G, gr, cells);
 }
 
 // _Pi (src/metric.jl:225-233): Pi_ab = rho u_a u_b + p delta_ab - tau_ab
@@ -107,10 +119,10 @@ __device__ __forceinline__ double metric_pi(const F* prim, const F* g, const F* 
 // dQ_c = 0; dQ_c -= inv_J D_d(A_d F_dc) for d = 1, 2, 3; then
 // add_metric_sources! (src/metric.jl:235-269) on the momentum components.
 template <typename F>
-__global__ void k_metric_div(F* __restrict__ dQ, const F* __restrict__ fd, int ncons, int Ns,
-                             const F* __restrict__ prim, const F* __restrict__ g, const F* __restrict__ art,
-                             double mu0, Geom G, Grid3 gr, int64_t cells) {
-    grid_dependency_wait();
+__device__ __forceinline__ void metric_div_body(F* __restrict__ dQ, const F* __restrict__ fd, int ncons, int Ns,
+                                                const F* __restrict__ prim, const F* __restrict__ g,
+                                                const F* __restrict__ art, double mu0, const Geom& G, const Grid3& gr,
+                                                int64_t cells) {
     GRID_STRIDE(I, cells) {
         int i, j, k;
         cell_ijk(I, gr.n, i, j, k);
@@ -138,6 +150,13 @@ __global__ void k_metric_div(F* __restrict__ dQ, const F* __restrict__ fd, int n
         }
         for (int a = 0; a < 3; ++a) dQ[I + cells * (Ns + a)] = F(mom[a]);
     }
+}
+template <typename F>
+__global__ void k_metric_div(F* dQ, const F* fd, int ncons, int Ns, const F* prim, const F* g, const F* art,
+                             double mu0, const __grid_constant__ Geom G, const __grid_constant__ Grid3 gr,
+                             int64_t cells) {
+    grid_dependency_wait();
+    metric_div_body<F>(dQ, fd, ncons, Ns, prim, g, art, mu0, G, gr, cells);
 }
 
 // max_rate per-block partials (src/timestep.jl:125-175) with the inverse

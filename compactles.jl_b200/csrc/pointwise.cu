@@ -163,12 +163,11 @@ __device__ __forceinline__ void rate_block_reduce(double rate, double rmin, doub
 // RATE: the max_rate reduction of the cells just formed, per-block partials into
 // part.  As a pass of its own it read seven of these fields again: 443 us of a
 // 256^3 FP64 step, 200 us of a 192^3 mixed one.
-template <typename F, bool N9, bool PM = false, bool RATE = false>
-__global__ void __launch_bounds__(kThreads, RATE ? 3 : 4) k_primitives(const double* __restrict__ Q, F* __restrict__ prim, int64_t cells, int Ns, PhysConst pc,
-                             int esens, const double* __restrict__ mc = nullptr, const int* __restrict__ tmap = nullptr,
-                             const F* __restrict__ art = nullptr, double* __restrict__ part = nullptr,
-                             const RateConst rc = RateConst{}) {
-    grid_dependency_wait();
+template <typename F, bool N9, bool PM, bool RATE>
+__device__ __forceinline__ void primitives_body(const double* __restrict__ Q, F* __restrict__ prim, int64_t cells,
+                                                int Ns, const PhysConst& pc, int esens, const double* __restrict__ mc,
+                                                const int* __restrict__ tmap, const F* __restrict__ art,
+                                                double* __restrict__ part, const RateConst& rc) {
     double rate = 0.0, rmin = __longlong_as_double(0x7ff0000000000000LL);
     GRID_STRIDE(I, cells) {
         const double* mcI = nullptr;
@@ -245,6 +244,14 @@ __global__ void __launch_bounds__(kThreads, RATE ? 3 : 4) k_primitives(const dou
     }
     if constexpr (RATE) rate_block_reduce(rate, rmin, part, blockIdx.x);
 }
+template <typename F, bool N9, bool PM = false, bool RATE = false>
+__global__ void __launch_bounds__(kThreads, RATE ? 3 : 4)
+    k_primitives(const double* Q, F* prim, int64_t cells, int Ns, const __grid_constant__ PhysConst pc, int esens,
+                 const double* mc = nullptr, const int* tmap = nullptr, const F* art = nullptr, double* part = nullptr,
+                 const __grid_constant__ RateConst rc = RateConst{}) {
+    grid_dependency_wait();
+    primitives_body<F, N9, PM, RATE>(Q, prim, cells, Ns, pc, esens, mc, tmap, art, part, rc);
+}
 
 // |S| = sqrt(S_ij S_ij) (src/artificial.jl:287-300); g[3d+j] = d u_j / d x_d.
 // DIMS: bit d set where the derivatives along d are not all zero (the others are
@@ -252,8 +259,7 @@ __global__ void __launch_bounds__(kThreads, RATE ? 3 : 4) k_primitives(const dou
 // A template: tested at run time the loads are no longer issued together (k_fluxes
 // on 256^3 FP64 cells 766 -> 1572 us).
 template <typename F, int DIMS>
-__global__ void k_strain(const F* __restrict__ g, F* __restrict__ out, int64_t cells) {
-    grid_dependency_wait();
+__device__ __forceinline__ void strain_body(const F* __restrict__ g, F* __restrict__ out, int64_t cells) {
     GRID_STRIDE(I, cells) {
         double gv[9];
 #pragma unroll
@@ -268,6 +274,11 @@ __global__ void k_strain(const F* __restrict__ g, F* __restrict__ out, int64_t c
             }
         out[I] = F(sqrt(ss));
     }
+}
+template <typename F, int DIMS>
+__global__ void k_strain(const F* g, F* out, int64_t cells) {
+    grid_dependency_wait();
+    strain_body<F, DIMS>(g, out, cells);
 }
 
 // delta4_sum! (src/artificial.jl:67-94): sum_d h_d^p |(1,-4,6,-4,1) f| along d,
@@ -485,29 +496,47 @@ __device__ __forceinline__ double compression_switch(const double* gv) {
 // mu*, beta* (optionally gated), kappa* and every D*_k from the smoothed sensors
 // (strain, internal energy, Y_1 ..; fields `cells` apart) in one pass
 // (src/artificial.jl:306-313, :334-341, :348-356).
-template <typename F>
-__global__ void k_art_coef(const F* __restrict__ sens, const F* __restrict__ prim, const F* __restrict__ g,
-                           F* __restrict__ art, int64_t cells, int Ns, double C_mu, double C_beta, double C_kappa,
-                           double C_D, int gate) {
-    grid_dependency_wait();
+template <typename F, bool SINGLE>
+__device__ __forceinline__ void art_coef_body(const F* __restrict__ sens, const F* __restrict__ prim,
+                                              const F* __restrict__ g, F* __restrict__ art, int64_t cells, int Ns,
+                                              double C_mu, double C_beta, double C_kappa, double C_D, int gate) {
     GRID_STRIDE(I, cells) {
+        // loads first: none moves above a store (256^3 FP64: 190 us with them in between, 153)
         const double rho = double(prim[I + cells * P_RHO]);
         const double c = double(prim[I + cells * P_C]);
+        const double T = double(prim[I + cells * P_T]);
         const double rs = rho * jl_max(double(sens[I]), 0.0);
+        const double se = jl_max(double(sens[I + cells]), 0.0);
+        F sy[4];
+        if constexpr (!SINGLE)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (e < Ns) sy[e] = sens[I + cells * (2 + e)];
         double beta = C_beta * rs;
         if (gate) {
             double gv[9];
             for (int k = 0; k < 9; ++k) gv[k] = double(g[I + cells * k]);
             beta *= compression_switch(gv);
         }
+        const double scale = rho * c / jl_max(T, 2.220446049250313e-16);
         art[I + cells * A_MU] = F(C_mu * rs);
         art[I + cells * A_BETA] = F(beta);
-        const double scale = rho * c / jl_max(double(prim[I + cells * P_T]), 2.220446049250313e-16);
-        art[I + cells * A_KAPPA] = F(C_kappa * scale * jl_max(double(sens[I + cells]), 0.0));
-        if (Ns > 1)
-            for (int sp = 0; sp < Ns; ++sp)
+        art[I + cells * A_KAPPA] = F(C_kappa * scale * se);
+        if constexpr (!SINGLE) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (e < Ns) art[I + cells * (A_D0 + e)] = F(C_D * c * jl_max(double(sy[e]), 0.0));
+            for (int sp = 4; sp < Ns; ++sp)
                 art[I + cells * (A_D0 + sp)] = F(C_D * c * jl_max(double(sens[I + cells * (2 + sp)]), 0.0));
+        }
     }
+}
+template <typename F, bool SINGLE>
+__global__ void __launch_bounds__(kThreads, sizeof(F) == 8 ? 5 : 6)
+    k_art_coef(const F* sens, const F* prim, const F* g, F* art, int64_t cells, int Ns, double C_mu, double C_beta,
+               double C_kappa, double C_D, int gate) {
+    grid_dependency_wait();
+    art_coef_body<F, SINGLE>(sens, prim, g, art, cells, Ns, C_mu, C_beta, C_kappa, C_D, gate);
 }
 
 // dilatation and switch for the :dilatation beta sensor (src/artificial.jl:208-218)
@@ -539,12 +568,12 @@ __global__ void k_beta_dilatation(const F* __restrict__ sensor, const F* __restr
 // stored, and off curvilinear grids (GEO adds curvature terms to them) its
 // gradients are zero and not read.  Two species on 2048 x 1024 cells: 169 us with
 // all three directions.
-template <typename F, bool SINGLE, bool N9, bool GEO, bool PM = false, int DIMS = 7>
-__global__ void k_fluxes(const double* __restrict__ Q, const F* __restrict__ prim, const F* __restrict__ g,
-                         const F* __restrict__ gty, const F* __restrict__ art, F* __restrict__ flux, int64_t cells,
-                         int Ns, PhysConst pc, double mu0, double Pr, double Sc, Geom G,
-                         const double* __restrict__ mc = nullptr, const int* __restrict__ tmap = nullptr) {
-    grid_dependency_wait();
+template <typename F, bool SINGLE, bool N9, bool GEO, bool PM, int DIMS>
+__device__ __forceinline__ void fluxes_body(const double* __restrict__ Q, const F* __restrict__ prim,
+                                            const F* __restrict__ g, const F* __restrict__ gty,
+                                            const F* __restrict__ art, F* __restrict__ flux, int64_t cells, int Ns,
+                                            const PhysConst& pc, double mu0, double Pr, double Sc, const Geom& G,
+                                            const double* __restrict__ mc, const int* __restrict__ tmap) {
     if (SINGLE) Ns = 1;
     const int ncons = Ns + 4;
     const int gstride = SINGLE ? 1 : 1 + Ns;
@@ -579,6 +608,13 @@ __global__ void k_fluxes(const double* __restrict__ Q, const F* __restrict__ pri
         const double t12 = mu * (gv[1] + gv[3]);
         const double t13 = mu * (gv[2] + gv[6]);
         const double t23 = mu * (gv[5] + gv[7]);
+        // Loaded ahead of the stores below, which no load moves above (256^3 FP64: 949 us
+        // a launch with these between the stores, 749 here; 192^3 FP32 213, 172).  After
+        // the stresses: loaded before them they cost 20 registers more.
+        F gT[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) gT[d] = (DIMS >> d) & 1 ? gty[I + cells * (int64_t)(d * gstride)] : F(0);
+        const F Y1 = SINGLE ? prim[I + cells * P_Y0] : F(1);
         const double tau[3][3] = {{t11, t12, t13}, {t12, t22, t23}, {t13, t23, t33}};
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -590,8 +626,7 @@ __global__ void k_fluxes(const double* __restrict__ Q, const F* __restrict__ pri
             F* fd = flux + cells * (int64_t)(d * ncons);
             double hdiff = 0.0;
             if (SINGLE) {
-                const double Yk = double(prim[I + cells * P_Y0]);
-                const double f0 = r * Yk * ud;
+                const double f0 = r * double(Y1) * ud;
                 fd[I] = F(CLES_AF(f0));
             } else {
                 double Vc = 0.0;
@@ -610,7 +645,7 @@ __global__ void k_fluxes(const double* __restrict__ Q, const F* __restrict__ pri
             const double m0 = r * ud * uv[0] + (d == 0 ? p : 0.0) - td[0];
             const double m1 = r * ud * uv[1] + (d == 1 ? p : 0.0) - td[1];
             const double m2 = r * ud * uv[2] + (d == 2 ? p : 0.0) - td[2];
-            const double en = (E + p) * ud - (uv[0] * td[0] + uv[1] * td[1] + uv[2] * td[2]) - ka * double(gd[I]) + hdiff;
+            const double en = (E + p) * ud - (uv[0] * td[0] + uv[1] * td[1] + uv[2] * td[2]) - ka * double(gT[d]) + hdiff;
             fd[I + cells * (Ns + 0)] = F(CLES_AF(m0));
             fd[I + cells * (Ns + 1)] = F(CLES_AF(m1));
             fd[I + cells * (Ns + 2)] = F(CLES_AF(m2));
@@ -618,6 +653,13 @@ __global__ void k_fluxes(const double* __restrict__ Q, const F* __restrict__ pri
         }
     }
 #undef CLES_AF
+}
+template <typename F, bool SINGLE, bool N9, bool GEO, bool PM = false, int DIMS = 7>
+__global__ void k_fluxes(const double* Q, const F* prim, const F* g, const F* gty, const F* art, F* flux,
+                         int64_t cells, int Ns, const __grid_constant__ PhysConst pc, double mu0, double Pr, double Sc,
+                         const __grid_constant__ Geom G, const double* mc = nullptr, const int* tmap = nullptr) {
+    grid_dependency_wait();
+    fluxes_body<F, SINGLE, N9, GEO, PM, DIMS>(Q, prim, g, gty, art, flux, cells, Ns, pc, mu0, Pr, Sc, G, mc, tmap);
 }
 
 // add_source!(::ConstantBodyForce) (src/sources.jl:42-65) for every body force
@@ -646,9 +688,8 @@ __global__ void k_body_forces(F* __restrict__ dQ, const double* __restrict__ Q, 
 
 // Low-storage RK update (src/timestep.jl:86-95): v = A du + dt dQ; du = v; Q += B v.
 template <typename F>
-__global__ void k_lsrk(double* __restrict__ Q, double* __restrict__ du, const F* __restrict__ dQ, int64_t n, double A,
-                       double B, double dt, const double* __restrict__ dtp) {
-    grid_dependency_wait();
+__device__ __forceinline__ void lsrk_body(double* __restrict__ Q, double* __restrict__ du, const F* __restrict__ dQ,
+                                          int64_t n, double A, double B, double dt, const double* __restrict__ dtp) {
     if (dtp) dt = *dtp;
     GRID_STRIDE(I, n) {
         const double v = A * du[I] + dt * double(dQ[I]);
@@ -656,9 +697,13 @@ __global__ void k_lsrk(double* __restrict__ Q, double* __restrict__ du, const F*
         Q[I] += B * v;
     }
 }
-
-__global__ void k_rate_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
+template <typename F>
+__global__ void k_lsrk(double* Q, double* du, const F* dQ, int64_t n, double A, double B, double dt, const double* dtp) {
     grid_dependency_wait();
+    lsrk_body<F>(Q, du, dQ, n, A, B, dt, dtp);
+}
+
+__device__ __forceinline__ void rate_final_body(const double* __restrict__ part, int nb, double* __restrict__ out) {
     __shared__ double sr[kThreads], sm[kThreads];
     double rate = 0.0, rmin = __longlong_as_double(0x7ff0000000000000LL);
     for (int b = threadIdx.x; b < nb; b += blockDim.x) {
@@ -676,6 +721,10 @@ __global__ void k_rate_final(const double* __restrict__ part, int nb, double* __
         __syncthreads();
     }
     if (threadIdx.x == 0) { out[0] = sr[0]; out[1] = sm[0]; }
+}
+__global__ void k_rate_final(const double* part, int nb, double* out) {
+    grid_dependency_wait();
+    rate_final_body(part, nb, out);
 }
 
 // Fixed-order sums (deterministic) for diagnostics: per-block partials then one block.
@@ -832,8 +881,7 @@ __global__ void k_bc_plane(double* __restrict__ Q, Grid3 g, int d, int side, int
 // them; its thread applies all of theirs in order (apply_bcs!, dimensions
 // ascending, low face first).  Six faces of a 129^3 box: 6 x 5 us as launches of
 // their own.
-__global__ void k_bc_faces(double* __restrict__ Q, Grid3 g, int Ns, const __grid_constant__ BcFaces F) {
-    grid_dependency_wait();
+__device__ __forceinline__ void bc_faces_body(double* __restrict__ Q, const Grid3& g, int Ns, const BcFaces& F) {
     const int f = blockIdx.y, d = F.d[f];
     const int64_t cells = (int64_t)g.n[0] * g.n[1] * g.n[2];
     const int o1 = d == 0 ? 1 : 0, o2 = d == 2 ? 1 : 2;
@@ -852,6 +900,10 @@ __global__ void k_bc_faces(double* __restrict__ Q, Grid3 g, int Ns, const __grid
         for (int e = f; e < F.n; ++e)
             if (on(e)) bc_cell(Q, I, cells, F.d[e], Ns, F.kind[e], F.st[e]);
     }
+}
+__global__ void k_bc_faces(double* Q, const __grid_constant__ Grid3 g, int Ns, const __grid_constant__ BcFaces F) {
+    grid_dependency_wait();
+    bc_faces_body(Q, g, Ns, F);
 }
 
 // correct_rhs!(::NSCBCOutflowBC) (src/nscbc.jl:59-157) and
@@ -1000,7 +1052,7 @@ __device__ __forceinline__ void clock_before_body(double* __restrict__ clk, cons
     clk[DC_DT_SEEN] = jl_max(clk[DC_DT_SEEN], dt);
     clk[DC_DT] = jl_min(dt, c.tfinal - clk[DC_T]);
 }
-__global__ void k_clock_before(double* __restrict__ clk, const double* __restrict__ rate_rmin, ClockConst c) {
+__global__ void k_clock_before(double* clk, const double* rate_rmin, ClockConst c) {
     grid_dependency_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     clock_before_body(clk, rate_rmin[0], rate_rmin[1], c);
@@ -1012,7 +1064,7 @@ __device__ __forceinline__ void clock_after_body(double* __restrict__ clk, const
     clk[DC_STEP] += 1.0;
     if (!(clk[DC_T] < c.tfinal) || !(clk[DC_STEP] < c.nmax)) clk[DC_DONE] = 1.0;
 }
-__global__ void k_clock_after(double* __restrict__ clk, ClockConst c) {
+__global__ void k_clock_after(double* clk, ClockConst c) {
     grid_dependency_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     clock_after_body(clk, c);
@@ -1219,7 +1271,10 @@ void Pointwise<F>::delta4_halo(const F* f0, const F* f1, F* o0, F* o1, const Gri
 template <typename F>
 void Pointwise<F>::art_coef(const F* sens, const F* prim, const F* g, F* art, int64_t cells, int Ns, double C_mu,
                             double C_beta, double C_kappa, double C_D, int gate, cudaStream_t st) {
-    LAUNCH_DEP(k_art_coef<F>, cells, st, sens, prim, g, art, cells, Ns, C_mu, C_beta, C_kappa, C_D, gate);
+    if (Ns == 1)
+        LAUNCH_DEP((k_art_coef<F, true>), cells, st, sens, prim, g, art, cells, Ns, C_mu, C_beta, C_kappa, C_D, gate);
+    else
+        LAUNCH_DEP((k_art_coef<F, false>), cells, st, sens, prim, g, art, cells, Ns, C_mu, C_beta, C_kappa, C_D, gate);
 }
 template <typename F>
 void Pointwise<F>::strain(const F* g, F* out, int64_t cells, int dims, cudaStream_t st) {

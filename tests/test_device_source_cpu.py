@@ -29,3 +29,47 @@ def test_cluster_barriers_order_memory(path):
         # one pair publishes the end values, a second one keeps them
         assert len(re.findall(r"ln_cluster_arrive\(\);", body)) == 2
         assert len(re.findall(r"ln_cluster_wait\(\);", body)) == 2
+
+
+def _kernels(code):
+    """(name, parameter list, body) of every __global__ function."""
+    for m in re.finditer(r"__global__", code):
+        i = code.index("(", m.end())
+        while True:   # attributes with arguments come before the name
+            depth, j = 0, i
+            while True:
+                depth += {"(": 1, ")": -1}.get(code[j], 0)
+                j += 1
+                if depth == 0:
+                    break
+            rest = code[j:].lstrip()
+            if rest.startswith("{"):
+                break
+            i = code.index("(", j)
+        b = code.index("{", j)
+        depth, e = 0, b
+        while True:
+            depth += {"{": 1, "}": -1}.get(code[e], 0)
+            e += 1
+            if depth == 0:
+                break
+        yield re.search(r"(\w+)\s*$", code[:i]).group(1), code[i + 1:j - 1], code[b:e]
+
+
+# tables of a plan: written before the plan's first launch and never again
+CONSTANT_TABLES = {"Gw", "Gg", "tab"}
+
+
+def test_dependent_kernels_promise_nothing_before_their_wait():
+    """A kernel that starts with grid_dependency_wait is alive while its predecessor
+    still writes.  `__restrict__` on its parameters would promise that nobody else
+    writes the memory while it lives, and let reads move above the wait."""
+    seen = 0
+    for path in SOURCES:
+        for name, params, body in _kernels(_code(path)):
+            if "grid_dependency_wait()" not in body:
+                continue
+            seen += 1
+            bad = [n for n in re.findall(r"__restrict__\s+(\w+)", params) if n not in CONSTANT_TABLES]
+            assert not bad, (path.name, name, bad)
+    assert seen >= 16
