@@ -223,6 +223,7 @@ struct LineArgs {
         double *Q, *du;
         double A, B, dt;
         const double* dtp;
+        int keep;
     } rk;
 };
 
@@ -278,6 +279,9 @@ struct RkEpilogue {
     double* du;
     double A, B, dt;
     const double* dtp;  // when set, dt is read from device memory (graph mode)
+    // k_line also stores dq into `out`: the right-hand side of a step's last stage,
+    // for cles_get_rhs (the tile kernels consume it)
+    int keep;
 };
 
 int num_sms();   // multiprocessors of the current device

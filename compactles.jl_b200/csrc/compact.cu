@@ -285,7 +285,7 @@ bool try_launch_line(const CompactPlan& plan, const FieldView& in, const FieldVi
     const int64_t st_in = plan.P.dim == 0 ? 1 : plan.P.dim == 1 ? in.sy : in.sz;
     const int64_t st_out = plan.P.dim == 0 ? 1 : plan.P.dim == 1 ? out.sy : out.sz;
     if (std::max(st_in, st_out) * 8 * 64 >= (int64_t)1 << 31) return false;
-    RkEpilogue rk{nullptr, nullptr, 0.0, 0.0, 0.0, nullptr};
+    RkEpilogue rk{nullptr, nullptr, 0.0, 0.0, 0.0, nullptr, 0};
     if (rkp) rk = *rkp;
     return (plan.dtype == CLES_F64 ? launch_line_f64 : launch_line_f32)(plan, in, out, count, mode, st, rk, rk_first, in2,
                                                                         out2, count2, num_sms());

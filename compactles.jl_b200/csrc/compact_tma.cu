@@ -1057,7 +1057,7 @@ bool try_launch_xt(const CompactPlan& plan, const FieldView& in, const FieldView
 
 bool try_launch_tma(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
                     cudaStream_t st, const RkEpilogue* rkp) {
-    RkEpilogue rk{nullptr, nullptr, 0.0, 0.0, 0.0, nullptr};
+    RkEpilogue rk{nullptr, nullptr, 0.0, 0.0, 0.0, nullptr, 0};
     if (rkp) rk = *rkp;
     if (mode == OUT_RK && !rkp) return false;
     if (!plan.has_tl && !plan.has_tg) return false;
@@ -1146,7 +1146,7 @@ bool try_launch_tg_split(const CompactPlan& plan, const FieldView& in, const Fie
                      base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return false;
-    const RkEpilogue rk{nullptr, nullptr, 0.0, 0.0, 0.0, nullptr};
+    const RkEpilogue rk{nullptr, nullptr, 0.0, 0.0, 0.0, nullptr, 0};
     if (plan.dtype == CLES_F64)
         return launch_tg<double>(plan, map, out, count, OUT_STORE, st, plan.tab64, rk, H, static_cast<double*>(iface));
     return launch_tg<float>(plan, map, out, count, OUT_STORE, st, plan.tab32, rk, H, static_cast<float*>(iface));

@@ -571,6 +571,7 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
                         for (int k = 0; k < 4; ++k)
                             if (i + 32 * k < ie) {
                                 const T dq = old[k] - src[i + 32 * k];
+                                if (A.rk.keep) row[i + 32 * k] = dq;
                                 const double v = A.rk.A * dv[k] + rdt * double(dq);
                                 dp[i + 32 * k] = v;
                                 Qp[i + 32 * k] = qv[k] + A.rk.B * v;
@@ -624,6 +625,7 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
                 for (int q = 0; q < 4; ++q)
                     if (i0 + q < m) {
                         const T dq = old[q] - y[i0 + q];
+                        if (A.rk.keep) at(i0 + q) = dq;
                         const double v = A.rk.A * dv[q] + rdt * double(dq);
                         atd(dp, i0 + q) = v;
                         atd(Qp, i0 + q) = qv[q] + A.rk.B * v;
@@ -713,7 +715,7 @@ void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView
     A.logL = 0;
     while ((1 << A.logL) < s.L) ++A.logL;
     A.mode = mode;
-    A.rk = {rk.Q, rk.du, rk.A, rk.B, rk.dt, rk.dtp};
+    A.rk = {rk.Q, rk.du, rk.A, rk.B, rk.dt, rk.dtp, rk.keep};
     A.rk_first = rk_first ? 1 : 0;
     A.pitch = 0;
     size_t smem = sizeof(T) * (size_t)s.SC * 2 * Q * s.L;

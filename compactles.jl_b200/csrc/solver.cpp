@@ -980,7 +980,7 @@ public:
             if (!first_prepared) apply_bcs();
             // the last flux-divergence direction applies the RK update in its
             // store when its plan takes the TMA path; otherwise a separate pass
-            const RkEpilogue rk{Q_.as<double>(), du_.as<double>(), RKA[stage], RKB[stage], dt};
+            const RkEpilogue rk{Q_.as<double>(), du_.as<double>(), RKA[stage], RKB[stage], dt, nullptr, stage == 4};
             if (!compute_rhs_impl(first_prepared, &rk))
                 Pointwise<F>::lsrk(Q_.as<double>(), du_.as<double>(), dQ_.as<F>(), cells_ * ncons_, RKA[stage],
                                    RKB[stage], dt, st_);
@@ -1253,7 +1253,7 @@ public:
             clock_before(clk, res_.as<double>(), cc_, st_);
             for (int stage = 0; stage < 5; ++stage) {
                 if (stage > 0) apply_bcs();
-                const RkEpilogue rk{Q_.as<double>(), du_.as<double>(), RKA[stage], RKB[stage], 0.0, clk + DC_DT};
+                const RkEpilogue rk{Q_.as<double>(), du_.as<double>(), RKA[stage], RKB[stage], 0.0, clk + DC_DT, stage == 4};
                 if (!compute_rhs_impl(stage == 0, &rk))
                     Pointwise<F>::lsrk(Q_.as<double>(), du_.as<double>(), dQ_.as<F>(), cells_ * ncons_, RKA[stage],
                                        RKB[stage], 0.0, st_, clk + DC_DT);

@@ -118,6 +118,34 @@ def test_rhs_and_steps(orc, n, walls):
     assert np.linalg.norm(qa - qb) < 1e-11 * np.linalg.norm(qb)
 
 
+@pytest.mark.parametrize("n", [(333, 1, 1), (150, 67, 1), (1, 61, 1), (45, 39, 51)])
+@pytest.mark.parametrize("graph", [False, True])
+def test_rhs_after_a_step(n, graph):
+    """The right-hand side read after a step is that of its last stage, also where
+    the update rides in the last direction's store.  A step of dt moves the stages by
+    dt d(dQ)/dt, here 1e-9 of dQ: frequencies of these grids are below 1e4, dt is
+    about 1e-13."""
+    import ctypes as C
+    d = cl.solver_desc(n, tuple(1.0 if v > 1 else 0.01 for v in n), cl.PER3, cl.lele_d1_6(), cl.compact_filter(0.45),
+                       cfl=1e-10)
+    tp = 2 * np.pi
+    Q0 = cl.initialize(d, lambda x, y, z: cl.Prim(
+        u=(0.3 * np.sin(tp * (x + y)) + 0 * z, 0.2 * np.cos(tp * x) + 0 * y + 0 * z, 0 * x + 0 * y + 0.1 * np.sin(tp * z)),
+        p=2 + 0.2 * np.sin(tp * (x + z)) + 0 * y, rho=1 + 0.1 * np.cos(tp * (y + z)) + 0 * x))
+    R, S = cl.Solver(d), cl.Solver(d)
+    R.set_state(Q0)
+    S.set_state(Q0)
+    ref = R.compute_rhs()
+    if graph:
+        S.run_graph(1.0, 1)
+    else:
+        S.step(1e-13)
+    got = np.full_like(ref, np.nan)
+    cl.api._check(cl.lib().cles_get_rhs(S.ptr, got.ctypes.data_as(C.c_void_p), S._layout("padded")))
+    sl = (slice(None),) + cl.interior_slices(d)
+    assert np.abs(got[sl] - ref[sl]).max() <= 1e-9 * np.abs(ref[sl]).max()
+
+
 @pytest.mark.parametrize("n", [(1, 61, 1), (41, 1, 38), (1, 44, 39)])
 def test_other_collapsed_dimensions(orc, n):
     """Grids whose collapsed dimension is not the last: every direction's code path runs."""
