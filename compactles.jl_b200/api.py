@@ -61,6 +61,8 @@ def lib():
         L.cles_ctx_destroy.argtypes = [vp]
         L.cles_ctx_set_stream.argtypes = [vp, vp]
         L.cles_selftest_bounded_wait.argtypes = [vp, C.c_int64]
+        L.cles_selftest_line_form.argtypes = [C.POINTER(abi.cles_grid), C.POINTER(abi.cles_scheme), C.c_int, C.c_int,
+                                              C.c_int, C.POINTER(C.c_int)]
         L.cles_plan_create.argtypes = [vp, C.POINTER(abi.cles_grid), C.POINTER(abi.cles_scheme), C.c_int, C.c_double,
                                        C.c_int, C.c_int, C.POINTER(vp)]
         L.cles_plan_destroy.argtypes = [vp]

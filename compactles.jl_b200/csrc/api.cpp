@@ -288,6 +288,27 @@ int cles_selftest_bounded_wait(cles_ctx* ctx, int64_t limit_ns) {
     API_END
 }
 
+int cles_selftest_line_form(const cles_grid* grid, const cles_scheme* scheme, int dim, int dtype, int count,
+                            int info[4]) {
+    API_BEGIN
+    if (!grid || !scheme || !info) throw Error(CLES_EINVAL, "null argument");
+    if (dim < 1 || dim > 3) throw Error(CLES_EINVAL, "dim must be 1, 2 or 3");
+    if (dtype != CLES_F64 && dtype != CLES_F32) throw Error(CLES_EINVAL, "dtype must be CLES_F64 or CLES_F32");
+    if (count < 1) throw Error(CLES_EINVAL, "count must be >= 1");
+    CompactPlan p;
+    build_compact_plan(p, *scheme, grid->n_global, dim - 1, grid->periodic[dim - 1] != 0, 1.0, dtype, 0, 0, false,
+                       false, 0, true);
+    info[0] = p.has_xw ? 1 : 0;
+    info[1] = info[2] = info[3] = 0;
+    if (p.line) {
+        const LineShape s = line_shape(p.P, *p.line, count, 148, dtype == CLES_F64 ? 8 : 4);
+        info[1] = p.line->S;
+        info[2] = p.line->MS;
+        info[3] = s.CL;
+    }
+    API_END
+}
+
 // ------------------------------------------------------------------ plans ----
 int cles_plan_create(cles_ctx* ctx, const cles_grid* grid, const cles_scheme* scheme, int dim, double h, int dtype,
                      int layout, cles_plan** out) {

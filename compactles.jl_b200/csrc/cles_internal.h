@@ -244,6 +244,12 @@ struct CompactPlan {
     ~CompactPlan();
 };
 
+// Launch shape of k_line: lines and segments per block, blocks per cluster.
+struct LineShape {
+    int L, SC, CL;
+};
+LineShape line_shape(const CompactParams& P, const LinePlan& lp, int count, int num_sms, size_t el);
+
 // Builds the plan of `scheme` along `dim` (0-based) of a grid with interior
 // extents n3[3]; periodic says whether the line wraps.  lo_fold / hi_fold set
 // a coordinate-singularity fold at that end of a closed line: the antipodal
@@ -251,9 +257,10 @@ struct CompactPlan {
 // lo_open / hi_open make that end of a non-periodic line a rank interface.
 // pow2_seg_max > 0 (batched plans): S is the fewest power-of-two segments of
 // at most pow2_seg_max (8, 16 or 32) points.
+// host_only: everything but the device tables (no CUDA call).
 void build_compact_plan(CompactPlan& plan, const cles_scheme& scheme, const int n3[3], int dim,
                         bool periodic, double h, int dtype, int lo_fold = 0, int hi_fold = 0,
-                        bool lo_open = false, bool hi_open = false, int pow2_seg_max = 0);
+                        bool lo_open = false, bool hi_open = false, int pow2_seg_max = 0, bool host_only = false);
 
 // The LHS band of one line (or one rank's piece of a split line), row-major
 // n x (2q+1): interior band, closure rows at closed ends, parity folds, and

@@ -652,46 +652,6 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
     if (CL > 1) ln_cluster_wait();
 }
 
-// Lines and segments per block.  Blocks of at most 256 threads (two or more per
-// SM): 32 lines each, 16 where that keeps a line in one block (x rows are
-// contiguous, and 16 FP64 y / z lanes still fill 128-byte rows; FP32 y / z lines
-// keep 32), else the line over a cluster of up to 8 blocks.  Fewer lines a block
-// where the launch would not fill the SMs twice: down to 8 (64-byte rows) along y
-// and z, 1 along x.  Where it cannot fill them once, a block that would have more
-// than 256 threads is cut into a cluster of 64-thread ones, whose SMs load and
-// solve side by side: 20 steps of a 5712-cell tube 5.84 ms as one block a line,
-// 5.73 as blocks of 256, 5.40 of 128, 4.90 of 64; lines of 1000 cells gain nothing
-// (8.6 us a launch, 9.6 cut).
-struct LineShape {
-    int L, SC, CL;
-};
-inline LineShape line_shape(const CompactParams& P, const LinePlan& lp, int count, int num_sms, size_t el) {
-    auto shape = [&](int L) {
-        LineShape s;
-        s.L = L;
-        s.CL = (lp.S * L + 255) / 256;
-        if (s.CL > 8) s.CL = 8;
-        s.SC = (lp.S + s.CL - 1) / s.CL;
-        s.CL = (lp.S + s.SC - 1) / s.SC;
-        return s;
-    };
-    const int lmin = P.dim == 0 ? 1 : 8;
-    int L = 32;
-    if (lp.S * L > 256 && (P.dim == 0 || el == 8)) L = 16;
-    while (L > lmin && L / 2 >= P.lines) L /= 2;
-    while (L > 1 && shape(L).SC * L > 512) L /= 2;
-    auto blocks = [&](int l) { return ((P.lines + l - 1) / l) * count * shape(l).CL; };
-    while (L > lmin && blocks(L) < 2 * num_sms) L /= 2;
-    LineShape s = shape(L);
-    if (blocks(L) < num_sms) {
-        const int threads = lp.S * L > 256 ? 64 : 256;
-        s.CL = std::min(8, (lp.S * L + threads - 1) / threads);
-        s.SC = (lp.S + s.CL - 1) / s.CL;
-        s.CL = (lp.S + s.SC - 1) / s.SC;
-    }
-    return s;
-}
-
 template <typename T, int Q, int M, int MS, bool XM>
 void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
                    cudaStream_t st, const RkEpilogue& rk, bool rk_first, const void* in2, void* out2, int count2, int num_sms) {

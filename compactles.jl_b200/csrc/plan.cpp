@@ -242,25 +242,40 @@ void pack_line_coef(LinePlan& lp, const CompactParams& P, const std::vector<doub
 // 22.5 / 12.8, 64^3 walls FP32 6.7 / 8.5.
 constexpr int64_t kLineWide = ((int64_t)1 << 18) + 1;
 
+// Segments of the line form of a plan of `lines` lines of n points along `dim`;
+// 0: none.  Two at least, at most 512 (eight blocks of 64), and long enough for the end
+// rows, the stencil and the closure rows' reads to stay within a segment and its halo
+// (base >= 9 > 16 - 8, see ln_group).  Few lines of more than 8192 points take the longer
+// tiles: a tube step at 8192 / 9001 / 12790 cells 0.25 / 0.27 / 0.31 ms in FP64, with the
+// generic kernel 1.16 / 1.16 / 1.91.
+int line_segments(int dim, int n, int64_t lines) {
+    constexpr int kMost = 512, kLeast = 9;
+    const bool wide = lines * n >= kLineWide && n > 32;
+    int tile = wide ? 32 : 16;
+    while (tile < 32 && (n + tile - 1) / tile > kMost) tile += 8;
+    int S = (n + tile - 1) / tile;
+    // Few x lines leave few lines a block, whose neighbouring threads read shared rows
+    // a segment length apart: an odd length keeps them on different banks, where the
+    // limits allow one (8192 cells: 16-point segments 0.254 ms a step, 23-point 0.261).
+    if (dim == 0 && !wide)
+        for (int s = S; s <= std::min(kMost, S + S / 4 + 1) && n / s >= kLeast; ++s) {
+            const int b = n / s, major = n % s > s / 2 ? b + 1 : b;
+            if (major & 1) {
+                S = s;
+                break;
+            }
+        }
+    return S < 2 || S > kMost || n / S < kLeast ? 0 : S;
+}
+
 void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
     const CompactParams& P = plan.P;
     const int n = P.n, q = P.q;
     const bool periodic = B.periodic;
     if (!((q == 1 && (P.M == 1 || P.M == 2 || P.M == 4)) || (q == 2 && P.M == 3))) return;
     auto lp = std::unique_ptr<LinePlan>(new LinePlan());
-    const bool wide = P.lines * n >= kLineWide && n > 32;
-    int S = (n + (wide ? 31 : 15)) / (wide ? 32 : 16);
-    // Short-tile x plans run few lines a block, whose neighbouring threads read
-    // shared rows a segment length apart: an odd length keeps them on different
-    // banks.
-    if (P.dim == 0 && !wide)
-        for (int s = S; s <= S + S / 4 + 1; ++s) {
-            const int b = n / s, major = n % s > s / 2 ? b + 1 : b;
-            if (major & 1) { S = s; break; }
-        }
-    // two segments at least, long enough for the end rows, the stencil and the
-    // closure rows' reads to stay within a segment and its halo
-    if (S < 2 || S > 512 || n / S < 9) return;   // base >= 9 > 16 - 8, see ln_group
+    const int S = line_segments(P.dim, n, P.lines);
+    if (S == 0) return;
     lp->S = S;
     lp->base = n / S;
     lp->rem = n % S;
@@ -504,6 +519,43 @@ void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
 
 }  // namespace
 
+// Lines and segments per block.  Blocks of at most 256 threads (two or more per
+// SM): 32 lines each, 16 where that keeps a line in one block (x rows are
+// contiguous, and 16 FP64 y / z lanes still fill 128-byte rows; FP32 y / z lines
+// keep 32), else the line over a cluster of up to 8 blocks.  Fewer lines a block
+// where the launch would not fill the SMs twice: down to 8 (64-byte rows) along y
+// and z, 1 along x.  Where it cannot fill them once, a block that would have more
+// than 256 threads is cut into a cluster of 64-thread ones, whose SMs load and
+// solve side by side: 20 steps of a 5712-cell tube 5.84 ms as one block a line,
+// 5.73 as blocks of 256, 5.40 of 128, 4.90 of 64; lines of 1000 cells gain nothing
+// (8.6 us a launch, 9.6 cut).
+LineShape line_shape(const CompactParams& P, const LinePlan& lp, int count, int num_sms, size_t el) {
+    auto shape = [&](int L) {
+        LineShape s;
+        s.L = L;
+        s.CL = (lp.S * L + 255) / 256;
+        if (s.CL > 8) s.CL = 8;
+        s.SC = (lp.S + s.CL - 1) / s.CL;
+        s.CL = (lp.S + s.SC - 1) / s.SC;
+        return s;
+    };
+    const int lmin = P.dim == 0 ? 1 : 8;
+    int L = 32;
+    if (lp.S * L > 256 && (P.dim == 0 || el == 8)) L = 16;
+    while (L > lmin && L / 2 >= P.lines) L /= 2;
+    while (L > 1 && shape(L).SC * L > 512) L /= 2;
+    auto blocks = [&](int l) { return ((P.lines + l - 1) / l) * count * shape(l).CL; };
+    while (L > lmin && blocks(L) < 2 * num_sms) L /= 2;
+    LineShape s = shape(L);
+    if (blocks(L) < num_sms) {
+        const int threads = lp.S * L > 256 ? 64 : 256;
+        s.CL = std::min(8, (lp.S * L + threads - 1) / threads);
+        s.SC = (lp.S + s.CL - 1) / s.CL;
+        s.CL = (lp.S + s.SC - 1) / s.SC;
+    }
+    return s;
+}
+
 CompactPlan::~CompactPlan() {
     if (dev) cudaFree(dev);
 }
@@ -589,7 +641,8 @@ void LineBand::solve(double* x) const {
 }
 
 void build_compact_plan(CompactPlan& plan, const cles_scheme& s, const int n3[3], int dim, bool periodic,
-                        double h, int dtype, int lo_fold, int hi_fold, bool lo_open, bool hi_open, int pow2_seg_max) {
+                        double h, int dtype, int lo_fold, int hi_fold, bool lo_open, bool hi_open, int pow2_seg_max,
+                        bool host_only) {
     const int n = n3[dim];
     const int q = s.q, M = s.M, nc = s.nc;
     if (q < 1 || q > CLES_MAX_Q) throw Error(CLES_EINVAL, "scheme LHS half-bandwidth q must be 1 or 2");
@@ -958,6 +1011,7 @@ void build_compact_plan(CompactPlan& plan, const cles_scheme& s, const int n3[3]
     plan.dtype = dtype;
     plan.tab_elems = (size_t)total;
     if (!lo_open && !hi_open && pow2_seg_max == 0) build_line_plan(plan, B, dtype);
+    if (host_only) return;
     // every table of the plan in one device block and one copy
     std::vector<unsigned char> blob;
     auto put = [&](const void* src, size_t bytes) {

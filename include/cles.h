@@ -173,6 +173,15 @@ int64_t cles_kernel_launches(void);
  * path works; the context stays usable. */
 int  cles_selftest_bounded_wait(cles_ctx* ctx, int64_t limit_ns);
 
+/* Self-test of the kernel choice for a directional plan (no counterpart in the
+ * reference; host only, no device needed).  info[0]: 1 when the plan has the
+ * warp-per-line form, which serves its x lines; info[1..3]: segments a line,
+ * register tile (points a segment at most) and blocks a cluster of the
+ * segmented line kernel over `count` fields on 148 multiprocessors, 0 when the
+ * plan has no such form (tile or generic kernels serve it). */
+int  cles_selftest_line_form(const cles_grid* grid, const cles_scheme* scheme, int dim, int dtype, int count,
+                             int info[4]);
+
 /* ---- directional plans ---------------------------------------------------
  * cles_plan_create replaces plan_direction(decomp, scheme, dim, h)
  * (src/operators.jl:44-101, src/operators_banded.jl:29-125): LHS assembly

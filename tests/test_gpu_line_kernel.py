@@ -26,8 +26,19 @@ def _scheme(mod, name):
             "pade": mod.pade_d1_4, "slow": lambda: mod.compact_filter(0.4995)}[name]()
 
 
-def _check(orc, name, ng, dim, periodic, dtype, tol):
+def _line_form(ng, name, dim, periodic, dtype, count=1):
+    """(warp-per-line form, segments a line, points a segment, blocks a cluster)"""
+    import ctypes as C
     per = tuple(1 if (k != dim - 1 or periodic) else 0 for k in range(3))
+    info = (C.c_int * 4)()
+    cl.api._check(cl.lib().cles_selftest_line_form(C.byref(cl.grid(ng, per)), C.byref(_scheme(cl, name)), dim,
+                                                   cl.abi.CLES_F64 if dtype == "f64" else cl.abi.CLES_F32, count, info))
+    return tuple(info)
+
+
+def _check(orc, name, ng, dim, periodic, dtype, tol, form=True):
+    per = tuple(1 if (k != dim - 1 or periodic) else 0 for k in range(3))
+    assert (_line_form(ng, name, dim, periodic, dtype)[1] > 0) == form   # k_line can take it
     g = orc.grid(ng, per)
     rng = np.random.default_rng(ng[dim - 1] + 10 * dim)
     f = np.zeros(orc.padded_shape(g))
@@ -54,7 +65,7 @@ def _check(orc, name, ng, dim, periodic, dtype, tol):
 @pytest.mark.parametrize("dim", [1, 2, 3])
 @pytest.mark.parametrize("periodic", [True, False])
 def test_lengths(orc, scheme, dim, periodic):
-    for n in (18, 20, 31, 32, 33, 47, 49, 63, 65, 97, 129, 161, 255, 257, 1031):
+    for n in (18, 20, 21, 31, 32, 33, 35, 47, 49, 63, 65, 97, 129, 161, 255, 257, 1031):
         ng = tuple(n if k == dim - 1 else (7, 5, 6)[k] + 4 for k in range(3))
         _check(orc, scheme, ng, dim, periodic, "f64", 1e-12)
         _check(orc, scheme, ng, dim, periodic, "f32", 5e-6)
@@ -64,7 +75,7 @@ def test_lengths(orc, scheme, dim, periodic):
 @pytest.mark.parametrize("dim", [1, 2, 3])
 @pytest.mark.parametrize("n", [33, 161, 200])
 def test_many_lines(orc, scheme, dim, n):
-    # enough points for the long tile: 2^21 and more
+    # enough points for the long tile (more than 2^18): 2^21 and more
     o = int(np.ceil(np.sqrt((1 << 21) / n))) + 1
     ng = tuple(n if k == dim - 1 else o for k in range(3))
     for periodic in (True, False):
@@ -72,7 +83,8 @@ def test_many_lines(orc, scheme, dim, n):
     _check(orc, scheme, ng, dim, False, "f32", 5e-6)
 
 
-@pytest.mark.parametrize("ng,dim", [((9001, 1, 1), 1), ((4099, 40, 1), 1), ((37, 4099, 1), 2), ((300, 2049, 1), 2)])
+@pytest.mark.parametrize("ng,dim", [((7937, 1, 1), 1), ((8192, 1, 1), 1), ((9001, 1, 1), 1), ((12800, 1, 1), 1),
+                                    ((12000, 16, 1), 1), ((3, 8999, 1), 2), ((4099, 40, 1), 1), ((37, 4099, 1), 2), ((300, 2049, 1), 2)])
 def test_lines_over_clusters(orc, ng, dim):
     for scheme in ("c6", "c10", "filt"):
         for periodic in (True, False):
@@ -80,9 +92,11 @@ def test_lines_over_clusters(orc, ng, dim):
 
 
 def test_slow_filter(orc):
-    for dim in (1, 2):
-        ng = tuple(300 if k == dim - 1 else 9 for k in range(3))
-        _check(orc, "slow", ng, dim, False, "f64", 1e-11)   # condition number of the filter about 2000
+    # 300 points: the window holds the whole line; 1000: no window is wide enough
+    for n, form in ((300, True), (1000, False)):
+        for dim in (1, 2):
+            ng = tuple(n if k == dim - 1 else 9 for k in range(3))
+            _check(orc, "slow", ng, dim, False, "f64", 1e-11, form)   # condition number of the filter about 2000
 
 
 @pytest.mark.parametrize("n", [(333, 1, 1), (150, 67, 1), (45, 39, 51), (129, 40, 33)])
