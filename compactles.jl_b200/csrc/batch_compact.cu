@@ -49,11 +49,8 @@ void launch_k(const BatchLaunchKind& k, const BatchLinePlan* plans, const int2* 
               void* out, int64_t ct, int count, int mode, double* Q_, double* du, double A, double B, int skip,
               cudaStream_t st) {
     auto kern = k_compact_batch<T, Q, M, X, MS>;
-    static thread_local size_t configured = 0;
-    if (k.smem > 48 * 1024 && configured < k.smem) {
-        CLES_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem));
-        configured = k.smem;
-    }
+    static std::atomic<uint64_t> raised{0};
+    raise_smem_limit(kern, k.smem, raised);
     dim3 grid((unsigned)nblocks, (unsigned)count);
     kern<<<grid, k.threads, k.smem, st>>>(plans, blocks, static_cast<const T*>(in), static_cast<T*>(out), ct, mode,
                                           Q_, du, A, B, skip);

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <atomic>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -78,6 +79,22 @@ inline void launch_dependent(void (*kern)(K...), dim3 grid, dim3 block, size_t s
         cfg.numAttrs = 1;
     }
     CLES_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...));
+}
+// A launch with more than 48 KB of dynamic shared memory needs the kernel's limit
+// raised.  The limit belongs to the kernel and device, not to a launch or a host
+// thread: it goes to the device's maximum once (`raised`: the kernel's devices), never
+// to one launch's size, which another thread's larger launch may be between its own
+// call and its launch.
+constexpr size_t kMaxDynamicSmem = 227 * 1024;   // sm_100, kernels without static shared memory
+template <typename K>
+inline void raise_smem_limit(K* kern, size_t bytes, std::atomic<uint64_t>& raised) {
+    if (bytes <= 48 * 1024) return;
+    int dev = 0;
+    CLES_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = dev < 64 ? (uint64_t)1 << dev : 0;
+    if (raised.load(std::memory_order_acquire) & bit) return;
+    CLES_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynamicSmem));
+    raised.fetch_or(bit, std::memory_order_release);
 }
 #endif
 

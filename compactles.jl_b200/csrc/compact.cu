@@ -219,11 +219,8 @@ void launch_t(const CompactParams& P, const T* tab, const FieldView& in, const F
     if (P.pcr) smem += sizeof(T) * (size_t)P.LB * 4 * P.S;
     else if (P.hasred) smem += sizeof(T) * (size_t)P.LB * (N + 1);
     auto kern = k_compact<T, Q, M, X, MS>;
-    static thread_local int configured = 0;
-    if (smem > 48 * 1024 && configured < (int)smem) {
-        CLES_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = (int)smem;
-    }
+    static std::atomic<uint64_t> raised{0};
+    raise_smem_limit(kern, smem, raised);
     dim3 grid((unsigned)((P.lines + P.LB - 1) / P.LB), (unsigned)count);
     dim3 block((unsigned)(P.LB * P.S));
     kern<<<grid, block, smem, st>>>(P, tab, in, out, mode, iface);

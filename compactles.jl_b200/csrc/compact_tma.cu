@@ -879,11 +879,8 @@ void launch_tma_ms(const CompactPlan& plan, const CUtensorMap& map, const FieldV
     if (per_sm == 2) NS = tiles_for_two_ctas(tile_bytes, extra);
     const size_t smem = tile_bytes * NS + extra;
     auto kern = k_compact_tma<T, M, MS, CPS>;
-    static int configured = 0;
-    if (configured < (int)smem) {
-        CLES_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = (int)smem;
-    }
+    static std::atomic<uint64_t> raised{0};
+    raise_smem_limit(kern, smem, raised);
     if (!g_num_sms) {
         int dev = 0;
         CLES_CUDA(cudaGetDevice(&dev));
@@ -926,11 +923,8 @@ void launch_tg_ms(const CompactPlan& plan, const CUtensorMap& map, const FieldVi
     const int NS = tiles_for_two_ctas(tile_bytes, extra);
     const size_t smem = tile_bytes * NS + extra;
     auto kern = k_compact_tg<T, Q, M, MS>;
-    static int configured = 0;
-    if (configured < (int)smem) {
-        CLES_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = (int)smem;
-    }
+    static std::atomic<uint64_t> raised{0};
+    raise_smem_limit(kern, smem, raised);
     if (!g_num_sms) {
         int dev = 0;
         CLES_CUDA(cudaGetDevice(&dev));
@@ -986,11 +980,8 @@ void launch_xt_ms(const CompactPlan& plan, const FieldView& in, const FieldView&
     const size_t smem = sizeof(T) * ((size_t)(P.n + 2 * H) * (kLanes + 1) * NS +
                                      (size_t)kLanes * (N + 1) + (size_t)N * N);
     auto kern = k_compact_xt<T, Q, M, MS, NS>;
-    static int configured = 0;
-    if (configured < (int)smem) {
-        CLES_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = (int)smem;
-    }
+    static std::atomic<uint64_t> raised{0};
+    raise_smem_limit(kern, smem, raised);
     if (!g_num_sms) {
         int dev = 0;
         CLES_CUDA(cudaGetDevice(&dev));

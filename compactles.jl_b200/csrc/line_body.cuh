@@ -694,8 +694,8 @@ void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView
         }
     }
     auto kern = k_line<T, Q, M, MS, XM>;
-    if (smem > 48 * 1024)
-        CLES_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static std::atomic<uint64_t> raised{0};
+    raise_smem_limit(kern, smem, raised);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((P.lines + s.L - 1) / s.L) * s.CL, (unsigned)(count + count2));
     // whole warps for the row copies; threads past SC segments only take part

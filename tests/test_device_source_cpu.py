@@ -1,5 +1,5 @@
-"""Rules on the order of memory accesses in the device code that no run can show
-to be broken: read from the sources.
+"""Rules on memory order and shared launch state that a run shows to be broken only
+by chance: read from the sources.
 """
 import pathlib
 import re
@@ -73,3 +73,17 @@ def test_dependent_kernels_promise_nothing_before_their_wait():
             bad = [n for n in re.findall(r"__restrict__\s+(\w+)", params) if n not in CONSTANT_TABLES]
             assert not bad, (path.name, name, bad)
     assert seen >= 16
+
+
+def test_shared_memory_limits_are_only_raised_to_the_maximum():
+    """A kernel's dynamic shared memory limit is shared by every plan and host thread of
+    a device: set to one launch's size, it may undercut a larger launch that another
+    thread is about to make.  It is set in one place, to the device's maximum."""
+    calls = []
+    for path in sorted(CSRC.iterdir()):
+        if path.suffix in (".cu", ".cuh", ".cpp", ".h"):
+            calls += [(path.name, m.group(1)) for m in
+                      re.finditer(r"cudaFuncSetAttribute\(([^;]*)\);", _code(path))]
+    assert [c[0] for c in calls] == ["cles_internal.h"], calls
+    assert calls[0][1].rstrip(")").endswith("(int)kMaxDynamicSmem"), calls
+    assert "kMaxDynamicSmem = 227 * 1024;" in _code(CSRC / "cles_internal.h")
