@@ -309,6 +309,8 @@ struct RkEpilogue {
 };
 
 int num_sms();   // multiprocessors of the current device
+// Whether a tile kernel can take `count` fields of this plan and view (y / z lines).
+bool tma_takes(const CompactPlan& plan, const FieldView& in, int count);
 // TMA-pipelined y/z launch; false when the plan or the views do not qualify.
 bool try_launch_tma(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
                     cudaStream_t st, const RkEpilogue* rk = nullptr);

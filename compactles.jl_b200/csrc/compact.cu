@@ -328,8 +328,12 @@ void launch_compact_pair(const CompactPlan& plan, const FieldView& in, const Fie
                          const FieldView& in2, const FieldView& out2, int count2, cudaStream_t st) {
     const bool same = in.comp_stride == in2.comp_stride && in.sy == in2.sy && in.sz == in2.sz &&
                       out.comp_stride == out2.comp_stride && out.sy == out2.sy && out.sz == out2.sz;
-    // (a profiled launch is bracketed by launch_compact)
-    if (same && !profiling() && count > 0 && count2 > 0 && plan.P.lines > 0 && !plan.has_xw && !tile_first(plan) &&
+    // lines that a tile kernel takes are solved group by group, all others that are
+    // not the warp-per-line kernel's by k_line (two species on 2048x1024 cells: 7.77 ms
+    // for two steps with the y gradients apart, 7.71 together); a profiled launch is
+    // bracketed by launch_compact
+    const bool tile = tile_first(plan) && (tma_takes(plan, in, count) || tma_takes(plan, in2, count2));
+    if (same && !profiling() && count > 0 && count2 > 0 && plan.P.lines > 0 && !plan.has_xw && !tile &&
         try_launch_line(plan, in, out, count, OUT_STORE, st, nullptr, false, in2.base, out2.base, count2))
         return;
     launch_compact(plan, in, out, count, OUT_STORE, st);

@@ -1046,11 +1046,7 @@ bool try_launch_xt(const CompactPlan& plan, const FieldView& in, const FieldView
     return launch_xt<float>(plan, in, out, count, mode, st, plan.tab32);
 }
 
-bool try_launch_tma(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
-                    cudaStream_t st, const RkEpilogue* rkp) {
-    RkEpilogue rk{nullptr, nullptr, 0.0, 0.0, 0.0, nullptr, 0};
-    if (rkp) rk = *rkp;
-    if (mode == OUT_RK && !rkp) return false;
+bool tma_takes(const CompactPlan& plan, const FieldView& in, int count) {
     if (!plan.has_tl && !plan.has_tg) return false;
     if (plan.P.lo_open || plan.P.hi_open) return false;   // split lines: try_launch_tg_split
     const CompactParams& P = plan.P;
@@ -1062,12 +1058,23 @@ bool try_launch_tma(const CompactPlan& plan, const FieldView& in, const FieldVie
         if (gx * (P.dim == 1 ? P.nz : P.ny) * count < num_sms()) return false;   // see try_launch_xt
     }
     if (plan.has_tl && (P.q != 1 || !P.periodic || P.M < 1 || P.M > 4 || P.M == 3)) return false;
-    PFN_cuTensorMapEncodeTiled_v12000 enc = encode_fn();
-    if (!enc) return false;
+    if (plan.has_tl && plan.TL.m != 32 && plan.TL.m != 16) return false;
+    if (!encode_fn()) return false;
     const size_t el = plan.dtype == CLES_F64 ? 8 : 4;
     // TMA needs a 16-byte aligned base and strides that are multiples of 16 bytes
     if ((uintptr_t)in.base % 16 || (in.sy * el) % 16 || (in.sz * el) % 16 || (in.comp_stride * el) % 16) return false;
-    if (in.comp_stride < (int64_t)P.nz * in.sz) return false;
+    return in.comp_stride >= (int64_t)P.nz * in.sz;
+}
+
+bool try_launch_tma(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
+                    cudaStream_t st, const RkEpilogue* rkp) {
+    RkEpilogue rk{nullptr, nullptr, 0.0, 0.0, 0.0, nullptr, 0};
+    if (rkp) rk = *rkp;
+    if (mode == OUT_RK && !rkp) return false;
+    if (!tma_takes(plan, in, count)) return false;
+    const CompactParams& P = plan.P;
+    PFN_cuTensorMapEncodeTiled_v12000 enc = encode_fn();
+    const size_t el = plan.dtype == CLES_F64 ? 8 : 4;
     CUtensorMap map;
     cuuint64_t dims[4] = {(cuuint64_t)P.nx, (cuuint64_t)P.ny, (cuuint64_t)P.nz, (cuuint64_t)count};
     cuuint64_t strides[3] = {(cuuint64_t)(in.sy * el), (cuuint64_t)(in.sz * el), (cuuint64_t)(in.comp_stride * el)};
@@ -1082,7 +1089,6 @@ bool try_launch_tma(const CompactPlan& plan, const FieldView& in, const FieldVie
         return launch_tg<float>(plan, map, out, count, mode, st, plan.tab32, rk);
     }
     const int M = P.M;
-    if (plan.TL.m != 32 && plan.TL.m != 16) return false;
     if (plan.dtype == CLES_F64) {
         const double* G = plan.tab64 + P.off_G;
         if (M == 1) return launch_tma_m<double, 1>(plan, map, out, count, mode, st, G, rk);

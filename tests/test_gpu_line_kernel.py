@@ -188,3 +188,20 @@ def test_mixed_faces_share_edges(orc):
         O.apply_bcs()
         a, b = S.get_state()[sl], O.get_state()[sl]
         assert np.abs(a - b).max() <= 1e-14 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("ny", [161, 300, 1031])
+def test_gradient_groups_share_launches_on_long_lines(ny):
+    """Velocity and scalar gradients along y ride in one launch wherever k_line serves
+    the lines, also from 160 points on, where no tile kernel takes these lengths: as many
+    launches a right-hand side as with 150 points."""
+    def launches(n):
+        d = cl.solver_desc((40, n, 1), (1.0, 1.0, 0.01), cl.PER3, cl.lele_d1_6(), cl.compact_filter(0.45))
+        S = cl.Solver(d)
+        S.set_state(cl.initialize(d, lambda x, y, z: cl.Prim(u=(0.1 * np.sin(2 * np.pi * y) + 0 * x + 0 * z,
+                                                                0 * x + 0 * y + 0 * z, 0 * x + 0 * y + 0 * z),
+                                                             p=2 + 0 * x + 0 * y + 0 * z, rho=1 + 0 * x + 0 * y + 0 * z)))
+        before = cl.kernel_launches()
+        S.compute_rhs(layout="interior")
+        return cl.kernel_launches() - before
+    assert launches(ny) == launches(150)
