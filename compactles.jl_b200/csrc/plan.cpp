@@ -440,6 +440,7 @@ void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
     std::vector<int> row_of(S);
     std::vector<Rows> rows;
     int Kr = 0;
+    const int most = 96 / b2;   // segments of a window; the dense or cyclic forms serve slower schemes better
     for (int K = 4;; K *= 2) {
         const bool whole = 2 * K + 1 >= S;
         rows.clear();
@@ -485,9 +486,11 @@ void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
             row_of[s] = e;
         }
         if (good || whole) break;
+        // rows that still weigh K segments away need a window of 2 K + 1 or more
+        if (S > most && 2 * K + 1 > most) return;
     }
     const int Wn = std::min(2 * Kr + 1, S);
-    if (Wn * b2 > 96) return;   // slowly decaying scheme: the dense or cyclic forms serve it better
+    if (Wn > most) return;
     lp->Wn = Wn;
     lp->Kr = Kr;
     std::vector<double> tab((size_t)S * b2 * Wn * b2, 0.0);

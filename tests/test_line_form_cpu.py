@@ -1,6 +1,7 @@
 """Which plans the segmented line kernel takes, and how it cuts their lines: the
 host side of the choice, without a device."""
 import ctypes as C
+import time
 
 import pytest
 
@@ -63,6 +64,22 @@ def test_what_other_kernels_serve():
     assert _form((1000, 9, 9), cl.compact_filter(0.4995))[1] == 0            # decays too slowly
     assert _form((300, 9, 9), cl.compact_filter(0.4995))[1] > 0              # the window holds the line
     assert _form((256, 64, 64), cl.lele_d1_6(), periodic=True)[0] == 1       # warp per line
+
+
+def test_schemes_without_a_line_form_are_refused_early():
+    """A window past its limit ends the search for one: planning a filter that decays over
+    thousands of points takes no longer than planning any other on the same lines (both
+    spend 0.1 s on the generic form's interface inverse; the search used to go on to the
+    inverse of the whole line, 1 s)."""
+    def seconds(alpha, expect):
+        best = 1e9
+        for _ in range(3):
+            t = time.perf_counter()
+            form = _form((8192, 1, 1), cl.compact_filter(alpha), periodic=True)
+            best = min(best, time.perf_counter() - t)
+        assert (form[1] > 0) == expect
+        return best
+    assert seconds(0.49999, False) < 3 * seconds(0.45, True)
 
 
 def test_bad_arguments_are_refused():
