@@ -240,7 +240,6 @@ struct LineArgs {
         double *Q, *du;
         double A, B, dt;
         const double* dtp;
-        int keep;
     } rk;
 };
 

@@ -212,7 +212,9 @@ __device__ __forceinline__ void ln_stage(T* dst, const T* src, int count) {
     for (int i = threadIdx.x; i < count; i += blockDim.x) ln_cp_async(dst + i, src + i);
 }
 
-template <typename T, int Q, int M, int MS, bool XM>
+// KEEP: the RK store that also writes dq (RkEpilogue::keep), an instantiation of its
+// own: as a run-time branch it added up to 360 bytes of spills to the FP32 forms.
+template <typename T, int Q, int M, int MS, bool XM, bool KEEP = false>
 __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant__ CompactParams P,
                                                        const __grid_constant__ LnParam<T, Q, MS> C,
                                                        const __grid_constant__ LineArgs A, const T* __restrict__ Gw) {
@@ -518,7 +520,7 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
     }
 
     // ---- store ----
-    const int mode = A.mode;
+    const int mode = KEEP ? OUT_RK : A.mode;
     const double rdt = mode == OUT_RK ? (A.rk.dtp ? *A.rk.dtp : A.rk.dt) : 0.0;
     if (XM) {
         // every thread has read its window (the barrier above): results go
@@ -571,7 +573,7 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
                         for (int k = 0; k < 4; ++k)
                             if (i + 32 * k < ie) {
                                 const T dq = old[k] - src[i + 32 * k];
-                                if (A.rk.keep) row[i + 32 * k] = dq;
+                                if (KEEP) row[i + 32 * k] = dq;
                                 const double v = A.rk.A * dv[k] + rdt * double(dq);
                                 dp[i + 32 * k] = v;
                                 Qp[i + 32 * k] = qv[k] + A.rk.B * v;
@@ -625,7 +627,7 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
                 for (int q = 0; q < 4; ++q)
                     if (i0 + q < m) {
                         const T dq = old[q] - y[i0 + q];
-                        if (A.rk.keep) at(i0 + q) = dq;
+                        if (KEEP) at(i0 + q) = dq;
                         const double v = A.rk.A * dv[q] + rdt * double(dq);
                         atd(dp, i0 + q) = v;
                         atd(Qp, i0 + q) = qv[q] + A.rk.B * v;
@@ -652,8 +654,8 @@ __global__ void __maxnreg__((ln_regs<T, M, MS>())) k_line(const __grid_constant_
     if (CL > 1) ln_cluster_wait();
 }
 
-template <typename T, int Q, int M, int MS, bool XM>
-void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
+template <typename T, int Q, int M, int MS, bool XM, bool KEEP>
+void launch_line_k(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
                    cudaStream_t st, const RkEpilogue& rk, bool rk_first, const void* in2, void* out2, int count2, int num_sms) {
     const CompactParams& P = plan.P;
     const LinePlan& lp = *plan.line;
@@ -675,7 +677,7 @@ void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView
     A.logL = 0;
     while ((1 << A.logL) < s.L) ++A.logL;
     A.mode = mode;
-    A.rk = {rk.Q, rk.du, rk.A, rk.B, rk.dt, rk.dtp, rk.keep};
+    A.rk = {rk.Q, rk.du, rk.A, rk.B, rk.dt, rk.dtp};
     A.rk_first = rk_first ? 1 : 0;
     A.pitch = 0;
     size_t smem = sizeof(T) * (size_t)s.SC * 2 * Q * s.L;
@@ -693,7 +695,7 @@ void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView
             smem += g;
         }
     }
-    auto kern = k_line<T, Q, M, MS, XM>;
+    auto kern = k_line<T, Q, M, MS, XM, KEEP>;
     static std::atomic<uint64_t> raised{0};
     raise_smem_limit(kern, smem, raised);
     cudaLaunchConfig_t cfg = {};
@@ -723,6 +725,15 @@ void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView
     CLES_CUDA(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kern), args));
     count_launch();
     check_launch("k_line");
+}
+
+template <typename T, int Q, int M, int MS, bool XM>
+void launch_line_t(const CompactPlan& plan, const FieldView& in, const FieldView& out, int count, int mode,
+                   cudaStream_t st, const RkEpilogue& rk, bool rk_first, const void* in2, void* out2, int count2, int num_sms) {
+    if (mode == OUT_RK && rk.keep)
+        launch_line_k<T, Q, M, MS, XM, true>(plan, in, out, count, mode, st, rk, rk_first, in2, out2, count2, num_sms);
+    else
+        launch_line_k<T, Q, M, MS, XM, false>(plan, in, out, count, mode, st, rk, rk_first, in2, out2, count2, num_sms);
 }
 
 template <typename T, int Q, int M, bool XM>
