@@ -213,7 +213,7 @@ __host__ __device__ inline size_t line_row_index(int MS, int S, int n, int e, in
     return MS == 16 ? (size_t)e * S + s : (size_t)s * n + e;
 }
 
-// Segmented form of a line of any length (k_line): S segments, the first `rem`
+// Segmented form of a line (k_line; line_segments gives the lengths): S segments, the first `rem`
 // of base + 1 points and the others of base, on register tiles of MS points.
 struct LinePlan {
     int MS = 32, S = 0, base = 0, rem = 0;
@@ -233,7 +233,7 @@ struct LineArgs {
     int split;
     int S, base, rem, mm, Wn, Kr;
     int logL, SC, CL;                 // lines (log2) and segments per block, blocks per cluster
-    int pitch, kpad;                  // shared row of an x line: pitch, one pad element every 2^kpad
+    int pitch;                        // shared row of an x line, elements
     int gstage;                       // the inverse rows are staged in shared memory
     int mode, rk_first;
     struct {

@@ -1,5 +1,6 @@
-// Segmented compact line solve for lines of any length along any dimension:
-// the kernel behind launch_line (line_f64.cu, line_f32.cu).
+// Segmented compact line solve for lines of 18 points and more along any dimension
+// (up to 512 segments: 8192 points in short tiles, 16384 in long ones): the kernel
+// behind launch_line (line_f64.cu, line_f32.cu).
 //
 // A thread owns one segment of at most MS points of one line in registers.
 // Lines are cut into S segments of base or base + 1 points, so only four kinds
@@ -10,7 +11,8 @@
 // neighbouring interface values it needs from the rows of the reduced inverse
 // cut to a window of Wn segments (the inverse decays like rho^points away from
 // the diagonal; what the window leaves out is below 2^-60 of the row's sum, in
-// FP32 plans 2^-34).
+// FP32 plans 2^-34).  A value that is not finite therefore reaches its window only,
+// where a solve with the whole inverse spreads it over the line.
 //
 // The segments of one line may be spread over a cluster of CL blocks, which
 // exchange end values through distributed shared memory: long lines then need
@@ -22,11 +24,11 @@
 // part), in FP32 instruction issue; small plans latency.  Against the kernels it
 // replaced (generic segments with table loads; two launches of pieces for few long
 // lines), us a launch on B200:
-//   C10, three FP64 201x161x129 fields, walls, x / y / z: 243 / 166 / 136 -> 98 / 80 / 72
-//   C6, five FP64 129^3 fields, walls: 154 / 86 / 86 -> 64 / 48 / 49
-//   C6, six FP64 2048x1024 fields, walls, x / y: 211 / 120 -> 69 / 69
-//   C8 filter, five FP32 256x192x160 fields, walls, x: 130 -> 99
-//   C6, six FP64 lines of 5712 points: 18.9 -> 10.7
+//   C10, three FP64 201x161x129 fields, walls, x / y / z: 243 / 166 / 136 -> 99 / 80 / 72
+//   C6, five FP64 129^3 fields, walls: 154 / 86 / 86 -> 66 / 48 / 49
+//   C6, six FP64 2048x1024 fields, walls, x / y: 211 / 120 -> 72 / 68
+//   C8 filter, five FP32 256x192x160 fields, walls, x: 130 -> 101
+//   C6, six FP64 lines of 5712 points: 18.9 -> 10.8
 //
 // XM = false (y, z lines): lanes are consecutive x, the window is read straight
 // from global memory.  XM = true (x lines): the block's rows are staged by
@@ -178,8 +180,10 @@ __device__ __forceinline__ void ln_correct(const K& C, const int mm, T (&y)[MS],
     }
 }
 
-// Registers a thread: 16 to 24 warps on an SM in FP64, 24 to 32 in FP32 (without
-// spills; the filter's wide stencil takes more).
+// Registers a thread: 16 to 24 warps on an SM in FP64, 24 to 32 in FP32.  The FP64
+// 24- and 32-point tiles and the FP32 x lines fit; bytes spilled (stores / loads): FP64
+// 16-point y / z tiles of C4, C6 and C10 56 / 48, 64 / 72 and 224 / 240 (their x lines up
+// to 28 / 44, the filter 12 / 12), FP32 y / z tiles of C10 up to 80 / 72, others 28 / 36.
 template <typename T, int M, int MS>
 constexpr int ln_regs() {
     return sizeof(T) == 8 ? (MS == 32 ? 128 : MS == 24 ? 104 : M <= 2 ? 80 : 96) : (MS == 32 ? 80 : 64);

@@ -202,7 +202,7 @@ void build_warp_line(CompactPlan& plan, const Band& B, const cles_scheme& s, int
     plan.has_xw = true;
 }
 
-// ---- line form of any length (k_line) --------------------------------------
+// ---- segmented line form (k_line) --------------------------------------
 
 template <typename T, int Q, int MS>
 void pack_line_coef(LinePlan& lp, const CompactParams& P, const std::vector<double> f[4][5], const std::vector<double> v[4][2],
@@ -522,8 +522,9 @@ void build_line_plan(CompactPlan& plan, const Band& B, int dtype) {
 
 }  // namespace
 
-// Lines and segments per block.  Blocks of at most 256 threads (two or more per
-// SM): 32 lines each, 16 where that keeps a line in one block (x rows are
+// Lines and segments per block.  Blocks of at most 256 threads (two or more per SM), of
+// up to 512 only where eight of 256 do not hold the lines (more than 2048 / L segments; in
+// FP64 long tiles such a block has an SM to itself): 32 lines each, 16 where that keeps a line in one block (x rows are
 // contiguous, and 16 FP64 y / z lanes still fill 128-byte rows; FP32 y / z lines
 // keep 32), else the line over a cluster of up to 8 blocks.  Fewer lines a block
 // where the launch would not fill the SMs twice: down to 8 (64-byte rows) along y

@@ -157,7 +157,10 @@ __device__ __forceinline__ void rate_block_reduce(double rate, double rmin, doub
 
 // _primitives!(::IdealMixture) (src/physics.jl:604-653) at the interior, and
 // _primitives!(::Nasa9Mixture) (src/physics.jl:501-570) when N9 (a separate
-// instantiation, so the ideal-gas kernel keeps its small register footprint).
+// instantiation, so the ideal-gas kernel keeps its small register footprint).  The
+// bound on the registers serves both: N9 spills 168 / 196 bytes under it (RATE 56 / 120),
+// but the latency of its FP64 Newton chain wants the warps: two species on 128^3 cells
+// 345 us a launch, 367 at three blocks an SM, 432 at two, 438 without a bound.
 // PM (batched solves): the species constants are per batch member, mc[24 m ..]
 // = R_k, cv_k, cp_k (8 each) of member m = tmap[cell / 64].
 // RATE: the max_rate reduction of the cells just formed, per-block partials into

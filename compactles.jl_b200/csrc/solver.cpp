@@ -978,8 +978,8 @@ public:
             tstage = t + RKC[stage] * dt;
             const bool first_prepared = prepared && stage == 0;
             if (!first_prepared) apply_bcs();
-            // the last flux-divergence direction applies the RK update in its
-            // store when its plan takes the TMA path; otherwise a separate pass
+            // the last flux-divergence direction applies the RK update in its store
+            // where a tile kernel or k_line takes its plan; otherwise a separate pass
             const RkEpilogue rk{Q_.as<double>(), du_.as<double>(), RKA[stage], RKB[stage], dt, nullptr, stage == 4};
             if (!compute_rhs_impl(first_prepared, &rk))
                 Pointwise<F>::lsrk(Q_.as<double>(), du_.as<double>(), dQ_.as<F>(), cells_ * ncons_, RKA[stage],

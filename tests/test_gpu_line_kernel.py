@@ -1,4 +1,4 @@
-"""Line solves of any length (k_line) against the CPU oracle.
+"""Segmented line solves (k_line) against the CPU oracle.
 
 Lengths on both sides of every boundary of the segmentation: tiles of 16, 24
 and 32 points, remainders (segments of two lengths), the smallest line with two

@@ -1,14 +1,13 @@
-"""Few long closed x lines, cut into pieces solved side by side on the device
-(SigPlan: the reference's P > 1 line solve, src/tridiag.jl:136-170 and
-src/banded.jl:177-214, with the pieces of one line in place of ranks).
+"""Few long closed x lines, spread over the blocks of a cluster (k_line: the
+reference's P > 1 line solve, src/tridiag.jl:136-170 and src/banded.jl:177-214,
+with segments of one line in place of ranks).
 
 The 1-D two-species shock tubes of the serving mix reach 8192 cells: one line
 per field.  Their right-hand side and steps of run! are compared with the CPU
-oracle (its single-rank Thomas solve) at lengths where the pieced form is
-used: FP64 per RHS within 1e-12 of the term scale and within 1e-10 relative
-L2 after 30 steps (host-stepped and graph mode), the mixed form within 1e-5;
-the C10 scheme and a thin 2-D grid of 3 long lines; and lengths on either
-side of the threshold (2047 and 2048 cells)."""
+oracle (its single-rank Thomas solve) at 2047 to 8192 cells: FP64 per RHS
+within 1e-12 of the term scale and within 1e-10 relative L2 after 30 steps
+(host-stepped and graph mode), the mixed form within 1e-5; the C10 scheme and
+a thin 2-D grid of 3 long lines."""
 import numpy as np
 import pytest
 
